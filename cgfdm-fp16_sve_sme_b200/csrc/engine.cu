@@ -5,7 +5,8 @@
 // device_common.cuh):
 //   A  wavefield at the start of a step; receives the step's result
 //   X, Y  RK stage ping-pong buffers
-//   T  RK4 accumulator
+//   T  RK4 accumulator (a whole step writes it in stage 2 only, see
+//      StageArgs::lean; stage() and the exact-order kernel in every stage)
 // Stage mapping: irk0 A->X, irk1 X->Y, irk2 Y->X, irk3 X->A, with the RK
 // "m" state read from A (it is the step-start wavefield for stages 0-2, the
 // reference's m_W copy, wave_rk.cpp:29).  PML auxiliaries use the same
@@ -235,7 +236,7 @@ template <typename S> class EngineT : public Engine {
     if (use_stream_) {
       S *bufs[3] = {A_, X_, Y_};
       for (int b = 0; b < 3; ++b) {
-        int rc = encode_stream_maps<S>(bufs[b], cjm_, A_, T_, g_.L, tmap_[b]);
+        int rc = encode_stream_maps<S>(bufs[b], cjm_, A_, T_, X_, g_.L, tmap_[b]);
         if (rc) return rc;
       }
     }
@@ -457,7 +458,7 @@ template <typename S> class EngineT : public Engine {
     for (int irk = 0; irk < 4 && !rc; ++irk) {
       int fb[3];
       step_fb(irk, fb);
-      rc = launch_stage(irk, fb, st);
+      rc = launch_stage(irk, fb, st, true);
     }
     return rc ? rc : step_end(st);
   }
@@ -487,7 +488,7 @@ template <typename S> class EngineT : public Engine {
     int fb[3] = {fb1, fb2, fb3};
     if (last_stream_ && last_stream_ != st) CUDA_TRY(cudaStreamSynchronize(last_stream_));
     last_stream_ = st;
-    return launch_stage(irk, fb, st);
+    return launch_stage(irk, fb, st, false);
   }
 
   int synchronize() override {
@@ -825,7 +826,9 @@ template <typename S> class EngineT : public Engine {
   }
 
   // Everything stage irk reads and writes (k range left to the caller).
-  StageArgs<S> stage_args(int irk, const int fb[3]) const {
+  // whole_step: a stage of run(); the exact-order kernel keeps the reference's
+  // accumulator there too.
+  StageArgs<S> stage_args(int irk, const int fb[3], bool whole_step) const {
     static const int in_of[4] = {0, 1, 2, 1}, out_of[4] = {1, 2, 1, 0};
     S *const bufs[3] = {A_, X_, Y_};
     StageArgs<S> a{};
@@ -842,6 +845,7 @@ template <typename S> class EngineT : public Engine {
     a.DT = d_.dt;
     a.fb1 = fb[0]; a.fb2 = fb[1]; a.fb3 = fb[2];
     a.irk = irk;
+    a.lean = whole_step && use_stream_ ? 1 : 0;
     a.chunk = chunk_;
     a.nslab = g_.npml > 0 ? 5 : 0;
     size_t off = 0;
@@ -868,7 +872,7 @@ template <typename S> class EngineT : public Engine {
   // only the step state A and step-start auxiliaries and writes X, T and the
   // stage-1 auxiliary inputs; stage 1 reads those and writes Y and T; the
   // real step rewrites all of them before reading them, so the timing leaves
-  // the run unchanged.  Results are cached per (precision, grid).
+  // the run unchanged (as stages of a whole step they leave T alone).  Results are cached per (precision, grid).
   // batch_form: a batch member, which always runs the 32 x 16 form inside
   // its batch; only the depth is chosen and the member's own form is kept.
   int tune(cudaStream_t st, bool batch_form = false) {
@@ -907,7 +911,7 @@ template <typename S> class EngineT : public Engine {
     cudaError_t err = cudaSuccess;
     for (int rows : forms)
       for (int ch : chunks) {
-        StageArgs<S> b0 = stage_args(0, fb0), b1 = stage_args(1, fb1);
+        StageArgs<S> b0 = stage_args(0, fb0, true), b1 = stage_args(1, fb1, true);
         b0.kbeg = b1.kbeg = HALO;
         b0.kend = b1.kend = g_.L.nz_ - HALO - 3;
         b0.chunk = b1.chunk = ch;
@@ -941,7 +945,7 @@ template <typename S> class EngineT : public Engine {
     float surf_ms[2] = {0, 0};
     for (int v = 0; v < 2 && err == cudaSuccess && !batch_form; ++v) {
       fast_top_ = v == 0;
-      const StageArgs<S> s0 = stage_args(0, fb0);
+      const StageArgs<S> s0 = stage_args(0, fb0, true);
       const int l0 = launches_;
       err = launch_surface(s0, st);
       if (err == cudaSuccess) err = cudaEventRecord(e0, st);
@@ -965,9 +969,9 @@ template <typename S> class EngineT : public Engine {
     return CGFDM_OK;
   }
 
-  int launch_stage(int irk, const int fb[3], cudaStream_t st) {
+  int launch_stage(int irk, const int fb[3], cudaStream_t st, bool whole_step) {
     static const int in_of[4] = {0, 1, 2, 1}, out_of[4] = {1, 2, 1, 0};
-    StageArgs<S> a = stage_args(irk, fb);
+    StageArgs<S> a = stage_args(irk, fb, whole_step);
     last_out_ = a.wout;
     last_aux_out_ = aux_total_ > 0 ? auxbuf(out_of[irk]) : nullptr;
     // events per timed stage: [0] start, [1] after the streaming kernel,
@@ -994,8 +998,9 @@ template <typename S> class EngineT : public Engine {
                                       tile_rows_ ? tile_rows_ : 16));
       if (ev) CUDA_TRY(cudaEventRecord(ev[2], st));
       // fields read and written per point by this stage: W in, 12 coefficients,
-      // W out, plus m (stages 1, 2) and t (written in 0, updated in 1-2, read in 3)
-      static const int nfield[4] = {39, 57, 57, 39};
+      // W out, plus m (stages 1, 2), stage 1's input (2) and t (written in 2,
+      // read in 3)
+      static const int nfield[4] = {30, 39, 57, 39};
       stream_bytes_ += (double)nfield[irk] * sizeof(S) * (double)(g_.nx) * g_.ny * (ksurf - HALO);
       CUDA_TRY(launch_surface(a, st));
     } else {
@@ -1039,7 +1044,7 @@ template <typename S> class EngineT : public Engine {
   // runs in a batch launch).
   int launch_top(int irk, const int fb[3], cudaStream_t st) {
     static const int out_of[4] = {1, 2, 1, 0};
-    StageArgs<S> a = stage_args(irk, fb);
+    StageArgs<S> a = stage_args(irk, fb, true);
     last_out_ = a.wout;
     last_aux_out_ = aux_total_ > 0 ? auxbuf(out_of[irk]) : nullptr;
     CUDA_TRY(launch_surface(a, st));
@@ -1293,7 +1298,7 @@ template <typename S> class BatchT : public BatchBase {
           int fb[3];
           m->step_fb(irk, fb);
           if (!m->use_stream_ || (fb[0] > 0) * 4 + (fb[1] > 0) * 2 + (fb[2] > 0) != code) continue;
-          StageArgs<S> a = m->stage_args(irk, fb);
+          StageArgs<S> a = m->stage_args(irk, fb, true);
           a.kbeg = HALO;
           a.kend = m->g_.L.nz_ - HALO - 3;
           args.push_back(a);
@@ -1306,7 +1311,7 @@ template <typename S> class BatchT : public BatchBase {
       for (auto *m : m_) {
         int fb[3];
         m->step_fb(irk, fb);
-        int rc = m->use_stream_ ? m->launch_top(irk, fb, st) : m->launch_stage(irk, fb, st);
+        int rc = m->use_stream_ ? m->launch_top(irk, fb, st) : m->launch_stage(irk, fb, st, true);
         if (rc) return rc;
       }
     }

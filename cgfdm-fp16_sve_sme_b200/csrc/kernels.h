@@ -27,7 +27,7 @@ template <typename S> cudaError_t launch_stage_top(const StageArgs<S> &a, cudaSt
 // TMA-staged z-streaming fused stage over kbeg <= k < kend, which must lie
 // below the three free-surface layers.  `maps` holds the tensor maps of the
 // stage input wavefield and of the coefficients (encode_stream_maps).
-constexpr int kStreamMapsBytes = 2048;
+constexpr int kStreamMapsBytes = 3072;
 // Tile form code of the paired-point kernel (16-bit storage): 64 x 8 tiles,
 // two x-adjacent points per thread.
 constexpr int kTilePair = 64;
@@ -53,11 +53,12 @@ cudaError_t launch_stage_stream_batch(const StageArgs<S> *args, const void *cons
 template <typename S> bool stage_stream_supported();
 // Encodes the tensor maps the streaming kernel loads its tiles through (the
 // 9 wavefield components of the stage input `wave`, the 13 coefficient
-// fields of `cjm`, the step state `wm` and the RK accumulator `t`) into `out`
-// (kStreamMapsBytes, 64-byte aligned host memory).
+// fields of `cjm`, the step state `wm`, the RK accumulator `t` and the stage
+// output `x`, which stage 2 of a whole step reads as stage 1's input) into
+// `out` (kStreamMapsBytes, 64-byte aligned host memory).
 template <typename S>
-int encode_stream_maps(const S *wave, const S *cjm, const S *wm, const S *t, const Layout &L,
-                       void *out);
+int encode_stream_maps(const S *wave, const S *cjm, const S *wm, const S *t, const S *x,
+                       const Layout &L, void *out);
 
 // Per-step values come from device memory so that a step can be replayed as
 // a CUDA graph: `step` points at the device step counter, advanced by the

@@ -156,7 +156,7 @@ int stage_noalloc(const cgfdm_stage_buffers &b, cudaStream_t st, unsigned char *
   const int ksurf = overlap ? HALO : L.nz_ - HALO - 3;
   if (ksurf > HALO) {  // the streaming launch has planes: it needs the tensor maps
     alignas(64) unsigned char maps[kStreamMapsBytes];
-    int rc = encode_stream_maps<S>(a.win, a.cjm, a.wm, a.t, L, maps);
+    int rc = encode_stream_maps<S>(a.win, a.cjm, a.wm, a.t, a.wout, L, maps);
     if (rc) return rc;
     StageArgs<S> lower = a;
     lower.kbeg = HALO;

@@ -248,17 +248,19 @@ __global__ void __launch_bounds__(256) stage_exact_kernel(StageArgs<S> a) {
       switch (a.irk) {
         case 0: {
           const R mv = ain[q];
-          at[q] = mv + (R)kB1 * hv;
+          if (!a.lean) at[q] = mv + (R)kB1 * hv;
           aout[q] = mv + (R)kA2rk * hv;
         } break;
         case 1:
-          at[q] = at[q] + (R)kB2 * hv;
+          if (!a.lean) at[q] = at[q] + (R)kB2 * hv;
           aout[q] = am[q] + (R)kA3rk * hv;
           break;
-        case 2:
-          at[q] = at[q] + (R)kB3 * hv;
-          aout[q] = am[q] + hv;
-          break;
+        case 2: {
+          const R mv = am[q];
+          at[q] = a.lean ? mv + ((R)kT1 * (aout[q] - mv) + ((R)kT2 * (ain[q] - mv) + (R)kB3 * hv))
+                         : at[q] + (R)kB3 * hv;
+          aout[q] = mv + hv;
+        } break;
         default:
           aout[q] = at[q] + (R)kB4 * hv;
       }
@@ -273,17 +275,22 @@ __global__ void __launch_bounds__(256) stage_exact_kernel(StageArgs<S> a) {
     switch (a.irk) {
       case 0: {
         const R mv = ldv(W + q);
-        stv(a.t + q, mv + (R)kB1 * hv);
+        if (!a.lean) stv(a.t + q, mv + (R)kB1 * hv);
         stv(a.wout + q, mv + (R)kA2rk * hv);
       } break;
       case 1: {
-        const R tv = ldv(a.t + q), mv = ldv(a.wm + q);
-        stv(a.t + q, tv + (R)kB2 * hv);
+        const R mv = ldv(a.wm + q);
+        if (!a.lean) stv(a.t + q, (R)ldv(a.t + q) + (R)kB2 * hv);
         stv(a.wout + q, mv + (R)kA3rk * hv);
       } break;
       case 2: {
-        const R tv = ldv(a.t + q), mv = ldv(a.wm + q);
-        stv(a.t + q, tv + (R)kB3 * hv);
+        const R mv = ldv(a.wm + q);
+        if (a.lean) {
+          const R w1 = ldv(a.wout + q), w2 = ldv(W + q);
+          stv(a.t + q, mv + ((R)kT1 * (w1 - mv) + ((R)kT2 * (w2 - mv) + (R)kB3 * hv)));
+        } else {
+          stv(a.t + q, (R)ldv(a.t + q) + (R)kB3 * hv);
+        }
         stv(a.wout + q, mv + hv);
       } break;
       default: {

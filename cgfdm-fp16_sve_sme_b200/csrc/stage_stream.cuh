@@ -14,8 +14,8 @@
 //   W ring (3): the 9 wavefield components of one input plane with the x/y
 //               halo of the one-sided stencils (x origin 16-byte aligned);
 //   C ring (2): the 9 metrics and (mu, lambda, buoyancy) of one output plane;
-//   M ring (2): the RK step state m and accumulator t of one output plane
-//               (stages that read them);
+//   M ring (2): the RK step state m and accumulator t (or what t is formed
+//               from) of one output plane (stages that read them);
 // (4/3/3 slots in the 16-bit PML variant, see Geo).
 // With 16-bit storage the interior variant converts each W plane to FP32 once
 // in shared memory (two plane buffers), so its stencils read FP32 like the
@@ -217,6 +217,16 @@ __device__ __forceinline__ float stencil1(float t0, float t1, float t2, float t3
   return fmaf(kA3, t4, fmaf(kA2, t3, fmaf(kA1, t2, fmaf(kA0, t1, kAm1 * t0))));
 }
 
+// t from the step state m, the inputs w1 and w2 of stages 1 and 2 and stage
+// 2's increment h (see StageArgs::lean).
+__device__ __forceinline__ float2 t_of_stages(float2 m, float2 w1, float2 w2, float cB, float2 h) {
+  const float2 nm = make_float2(-m.x, -m.y);
+  float2 s = __fmul2_rn(pk(cB), h);
+  s = __ffma2_rn(pk(kT2), __fadd2_rn(w2, nm), s);
+  s = __ffma2_rn(pk(kT1), __fadd2_rn(w1, nm), s);
+  return __fadd2_rn(m, s);
+}
+
 __device__ __forceinline__ unsigned slab_pos(const SlabDev<float> &sl, int i, int j, int k) {
   return (unsigned)((i - sl.off0) + (j - sl.off1) * sl.n0 + (k - sl.off2) * sl.n0 * sl.n1);
 }
@@ -228,8 +238,10 @@ __device__ __forceinline__ unsigned slab_pos(const SlabDev<float> &sl, int i, in
 // the slab, touch consecutive addresses.
 //
 // A point's inputs are the auxiliary input (part 1), what the stage adds the
-// increment to (part 2: m in stages 1-2, t in stage 3) and t (part 4, stages
-// 1-2).  pml_load<RK> loads the parts in a mask for all nine fields, so that
+// increment to (part 2: m in stages 1-2, t in stage 3) and what t comes from
+// (part 4, stages 1-2; tsel: kTsAcc = t itself, kTsNone = no t in this stage,
+// kTsOld = stage 1's input, which the output buffer still holds, see
+// StageArgs::lean).  pml_load<RK> loads the parts in a mask for all nine fields, so that
 // the loads can be issued at the top of a plane iteration and their latency
 // overlaps the stencil work; pml_apply<RK> is told which parts are already
 // in registers (a compile-time or a per-thread mask), loads the others
@@ -238,47 +250,55 @@ template <int RK> constexpr int pml_parts() { return RK == 0 ? 1 : RK == 3 ? 3 :
 struct PmlIn {
   float a[9], b[9], t[9];
 };
+enum { kTsAcc = 0, kTsNone = 1, kTsOld = 2 };
 template <int RK>
 __device__ __forceinline__ void pml_load_fields(const SlabDev<float> &sl, unsigned pos, int v0,
-                                                int nv, int mask, PmlIn &in) {
+                                                int nv, int mask, int tsel, PmlIn &in) {
   constexpr int P = pml_parts<RK>();
   const unsigned np = (unsigned)sl.np;
+  const float *tp = tsel == kTsOld ? sl.aout : sl.at;
 #pragma unroll
   for (int v = v0; v < v0 + nv; ++v) {
     const unsigned q = v * np + pos;
     if ((P & 1) && (mask & 1)) in.a[v] = sl.ain[q];
     if ((P & 2) && (mask & 2)) in.b[v] = RK == 3 ? sl.at[q] : sl.am[q];
-    if ((P & 4) && (mask & 4)) in.t[v] = sl.at[q];
+    if ((P & 4) && (mask & 4) && tsel != kTsNone) in.t[v] = tp[q];
   }
 }
 template <int RK>
-__device__ __forceinline__ void pml_load(const SlabDev<float> &sl, unsigned pos, int mask, PmlIn &in) {
-  pml_load_fields<RK>(sl, pos, 0, 9, mask, in);
+__device__ __forceinline__ void pml_load(const SlabDev<float> &sl, unsigned pos, int mask, int tsel,
+                                         PmlIn &in) {
+  pml_load_fields<RK>(sl, pos, 0, 9, mask, tsel, in);
 }
 // L1 prefetch of the parts in a mask (no registers held), for the parts the
 // stage needs but does not keep in registers across the stencils.
 template <int RK>
-__device__ __forceinline__ void pml_prefetch(const SlabDev<float> &sl, unsigned pos, int mask) {
+__device__ __forceinline__ void pml_prefetch(const SlabDev<float> &sl, unsigned pos, int mask,
+                                             int tsel) {
   constexpr int P = pml_parts<RK>();
   const unsigned np = (unsigned)sl.np;
+  const float *tp = tsel == kTsOld ? sl.aout : sl.at;
 #pragma unroll
   for (int v = 0; v < 9; ++v) {
     const unsigned q = v * np + pos;
     if ((P & 2) && (mask & 2))
       asm volatile("prefetch.global.L1 [%0];" ::"l"(RK == 3 ? sl.at + q : sl.am + q));
-    if ((P & 4) && (mask & 4)) asm volatile("prefetch.global.L1 [%0];" ::"l"(sl.at + q));
+    if ((P & 4) && (mask & 4) && tsel != kTsNone)
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(tp + q));
   }
 }
 template <int RK>
 __device__ __forceinline__ void pml_apply(const SlabDev<float> &sl, unsigned pos, const float E[9],
                                           float dl, float ad, float bt, float DT, float cB,
-                                          float cA, float h[9], int held, PmlIn &in) {
+                                          float cA, float h[9], int held, int tsel, int lean,
+                                          PmlIn &in) {
   const unsigned np = (unsigned)sl.np;
-  float *__restrict__ aout = sl.aout;
-  float *__restrict__ at = sl.at;
+  // (not __restrict__: with kTsOld part 4 is read through aout as well)
+  float *aout = sl.aout;
+  float *at = sl.at;
 #pragma unroll
   for (int g = 0; g < 9; g += 3) {
-    pml_load_fields<RK>(sl, pos, g, 3, 7 & ~held, in);
+    pml_load_fields<RK>(sl, pos, g, 3, 7 & ~held, tsel, in);
 #pragma unroll
     for (int v = g; v < g + 3; ++v) {
       const unsigned q = v * np + pos;
@@ -286,11 +306,13 @@ __device__ __forceinline__ void pml_apply(const SlabDev<float> &sl, unsigned pos
       const float ha = (dl * E[v] - ad * a) * DT;
       h[v] -= bt * a * DT;
       if (RK == 0) {
-        at[q] = a + kB1 * ha;
+        if (!lean) at[q] = a + kB1 * ha;
         aout[q] = a + kA2rk * ha;
       } else if (RK == 1) {
-        at[q] = in.t[v] + cB * ha;
-        aout[q] = in.b[v] + cA * ha;
+        const float m = in.b[v];
+        if (tsel == kTsAcc) at[q] = in.t[v] + cB * ha;
+        if (tsel == kTsOld) at[q] = m + (kT1 * (in.t[v] - m) + (kT2 * (a - m) + cB * ha));
+        aout[q] = m + cA * ha;
       } else {
         aout[q] = in.b[v] + kB4 * ha;
       }
@@ -310,6 +332,7 @@ struct Maps {
   CUtensorMap c3;  // coefficients, box 32 x TY x 1 x 3 (mu, lambda, b at field 10)
   CUtensorMap m;   // step-start wavefield, box 32 x TY x 1 x 9
   CUtensorMap t;   // RK accumulator, box 32 x TY x 1 x 9
+  CUtensorMap x;   // stage output before the stage, box 32 x TY x 1 x 9
 };
 struct MapSet {
   Maps ty16, ty8;  // the same buffers, boxes for tile heights 16 and 8
@@ -464,8 +487,12 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
     const Maps &maps = src.maps(e);
     const Work &wk = src.work(e);
     const Layout L = a.L;
-    // stages 1 and 2 (RK = 1) differ only in the weights of the t and output updates
-    constexpr bool need_m = RK == 1, need_t = RK >= 1;
+    // stages 1 and 2 (RK = 1) differ in the weights of the t and output
+    // updates and, in a whole step (a.lean), in what t comes from
+    constexpr bool ring_m = RK >= 1, need_m = RK == 1;
+    const int lean = a.lean;
+    const int tsel = RK != 1 || !lean ? kTsAcc : a.irk == 2 ? kTsOld : kTsNone;
+    const bool need_t = RK >= 1 && tsel != kTsNone;
     const float cB = a.irk == 2 ? kB3 : kB2, cA = a.irk == 2 ? 1.0f : kA3rk;
     const uint32_t m_bytes = (need_m ? 9 : 0) * NTHR * G::ES + (need_t ? 9 : 0) * NTHR * G::ES;
     const float rDH = a.rDH, DT = a.DT;
@@ -509,12 +536,14 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
       unsigned char *dst = smem + G::OFF_M + s * G::M_BYTES;
       mbar_expect_tx(bar, m_bytes);
       if (need_m) tma_load_4d(smem_u32(dst), &maps.m, tx0, ty0, k, 0, bar);
-      if (need_t) tma_load_4d(smem_u32(dst + 9 * NTHR * G::ES), &maps.t, tx0, ty0, k, 0, bar);
+      if (need_t)
+        tma_load_4d(smem_u32(dst + 9 * NTHR * G::ES), tsel == kTsOld ? &maps.x : &maps.t, tx0, ty0,
+                    k, 0, bar);
     };
     if (tid == 0) {
       for (int n = 0; n < NW - 1 && n < nplanes; ++n) issue_w(n);
       for (int o = 0; o < NC && o < nout; ++o) issue_c(o);
-      if (need_t)
+      if (ring_m)
         for (int o = 0; o < NM && o < nout; ++o) issue_m(o);
     }
 
@@ -573,14 +602,15 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
         sh = sx >= 0 ? sx : sy >= 0 ? sy : kk < HALO + a.npml ? 2 : -1;
         if (sh >= 0) {
           const unsigned pos = slab_pos(a.slab[sh], i, j, kk);
-          pml_load<RK>(a.slab[sh], pos, HP, pin);
-          if (HP != pml_parts<RK>()) pml_prefetch<RK>(a.slab[sh], pos, pml_parts<RK>() & ~HP);
+          pml_load<RK>(a.slab[sh], pos, HP, tsel, pin);
+          if (HP != pml_parts<RK>())
+            pml_prefetch<RK>(a.slab[sh], pos, pml_parts<RK>() & ~HP, tsel);
         }
       }
       bool ok = mbar_wait_bounded(smem_u32(&bw[(fw0 + n) % NW]), ((fw0 + n) / NW) & 1);
       if (o >= 0) {
         ok = ok && mbar_wait_bounded(smem_u32(&bc[(fc0 + o) % NC]), ((fc0 + o) / NC) & 1);
-        if (need_t) ok = ok && mbar_wait_bounded(smem_u32(&bm[(fm0 + o) % NM]), ((fm0 + o) / NM) & 1);
+        if (ring_m) ok = ok && mbar_wait_bounded(smem_u32(&bm[(fm0 + o) % NM]), ((fm0 + o) / NM) & 1);
       }
       // Every thread waits on the ring barriers itself, so no block barrier is
       // needed before the plane is read; a thread whose wait expired skips the
@@ -655,7 +685,8 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
         if constexpr (PMLK) {
           if (sx >= 0) {  // profile values d, alpha + d, beta at this x
             elastic9(mx, Lr, mu, lam, bu, E);
-            pml_apply<RK>(a.slab[sx], slab_pos(a.slab[sx], i, j, k), E, dlx, adx, btx, DT, cB, cA, pc, HP, pin);
+            pml_apply<RK>(a.slab[sx], slab_pos(a.slab[sx], i, j, k), E, dlx, adx, btx, DT, cB, cA, pc, HP, tsel,
+                          lean, pin);
           }
         }
         // y direction
@@ -679,7 +710,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
           if (sy >= 0) {
             elastic9(my, Lr, mu, lam, bu, E);
             pml_apply<RK>(a.slab[sy], slab_pos(a.slab[sy], i, j, k), E, dly, ady, bty, DT, cB, cA, pc,
-                          sh == sy ? HP : 0, pin);
+                          sh == sy ? HP : 0, tsel, lean, pin);
           }
         }
         // z direction: W[k - m*DIR] for m = -1..3 sits in slots P0 (q = k + DIR) .. P4
@@ -699,7 +730,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
             elastic9(mz, Lr, mu, lam, bu, E);
             const float d = __ldg(pz + 2 * L.nz_ + k), btz = __ldg(pz + L.nz_ + k), adz = __ldg(pz + k) + d;
             pml_apply<RK>(a.slab[2], slab_pos(a.slab[2], i, j, k), E, d * gz, adz, btz, DT, cB, cA, pc,
-                          sh == 2 ? HP : 0, pin);
+                          sh == 2 ? HP : 0, tsel, lean, pin);
           }
         }
         es.finish(mu, lam, bu, h);
@@ -711,7 +742,8 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
         }
         // RK4 combination (wave_rk.cpp:13-99), two fields at a time:
         // stage 0: t = m + B1 h, out = m + A2 h (the stage input at k is the step state m);
-        // stages 1-2: t += B h, out = m + A h; stage 3: out = t + B4 h
+        // stages 1-2: t += B h, out = m + A h; stage 3: out = t + B4 h;
+        // in a whole step only stage 2 writes t, see StageArgs::lean
         const S *ms = (const S *)(smem + G::OFF_M + ((fm0 + o) % NM) * G::M_BYTES);
         const S *ts = ms + 9 * NTHR;
         const long long ctr = L.at(i, j, k);
@@ -723,10 +755,12 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
           const float2 hv = pk(h[v], two ? h[v + 1] : 0.0f);
           const long long q = ctr + v * fs;
           float2 base_t, base_o;  // what t and the output add the increment to
+          base_t = pk(0.0f);
           if (RK == 0) {
             base_t = base_o = pk(win[v][P1], two ? win[v + 1][P1] : 0.0f);
           } else if (RK == 1) {
-            base_t = pk(ldv(ts + v * NTHR + cidx), two ? ldv(ts + (v + 1) * NTHR + cidx) : 0.0f);
+            if (need_t)
+              base_t = pk(ldv(ts + v * NTHR + cidx), two ? ldv(ts + (v + 1) * NTHR + cidx) : 0.0f);
             base_o = pk(ldv(ms + v * NTHR + cidx), two ? ldv(ms + (v + 1) * NTHR + cidx) : 0.0f);
           } else {
             base_o = pk(ldv(ts + v * NTHR + cidx), two ? ldv(ts + (v + 1) * NTHR + cidx) : 0.0f);
@@ -734,8 +768,11 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
           const float2 wo = __ffma2_rn(pk(cO), hv, base_o);
           stv(a.wout + q, wo.x);
           if (two) stv(a.wout + q + fs, wo.y);
-          if (RK <= 1) {
-            const float2 wt = __ffma2_rn(pk(cT), hv, base_t);
+          if (RK == 0 ? !lean : RK == 1 && need_t) {
+            const float2 wt =
+                RK == 1 && tsel == kTsOld
+                    ? t_of_stages(base_o, base_t, pk(win[v][P1], two ? win[v + 1][P1] : 0.0f), cT, hv)
+                    : __ffma2_rn(pk(cT), hv, base_t);
             stv(a.t + q, wt.x);
             if (two) stv(a.t + q + fs, wt.y);
           }
@@ -747,7 +784,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
       if (tid == 0) {
         if (n + NW - 1 < nplanes) issue_w(n + NW - 1);
         if (o >= 0 && o + NC < nout) issue_c(o + NC);
-        if (o >= 0 && need_t && o + NM < nout) issue_m(o + NM);
+        if (o >= 0 && ring_m && o + NM < nout) issue_m(o + NM);
       }
       return true;
     };
@@ -787,7 +824,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
         const int o = n - 4 > 0 ? n - 4 : 0;
         for (int m = o; m < nout && m < o + NC; ++m)
           mbar_wait_bounded(smem_u32(&bc[(fc0 + m) % NC]), ((fc0 + m) / NC) & 1);
-        if (need_t)
+        if (ring_m)
           for (int m = o; m < nout && m < o + NM; ++m)
             mbar_wait_bounded(smem_u32(&bm[(fm0 + m) % NM]), ((fm0 + m) / NM) & 1);
       }
@@ -795,7 +832,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
     }
     fw0 += nplanes;
     fc0 += nout;
-    if (need_t) fm0 += nout;
+    if (ring_m) fm0 += nout;
   }
 }
 
@@ -929,7 +966,10 @@ __global__ void __launch_bounds__(256, 1)
 
   unsigned fw0 = 0, fc0 = 0, fm0 = 0;  // ring fill counters, continued across items
   const Layout L = a.L;
-  constexpr bool need_m = RK == 1, need_t = RK >= 1;
+  constexpr bool ring_m = RK >= 1, need_m = RK == 1;
+  const int lean = a.lean;  // see StageArgs::lean and the one-point kernel
+  const int tsel = RK != 1 || !lean ? kTsAcc : a.irk == 2 ? kTsOld : kTsNone;
+  const bool need_t = RK >= 1 && tsel != kTsNone;
   const float cB = a.irk == 2 ? kB3 : kB2, cA = a.irk == 2 ? 1.0f : kA3rk;
   const uint32_t m_bytes = ((need_m ? 9 : 0) + (need_t ? 9 : 0)) * PLANE * 2;
   const float rDH = a.rDH, DT = a.DT;
@@ -977,12 +1017,14 @@ __global__ void __launch_bounds__(256, 1)
       unsigned char *dst = smem + G::OFF_M + q * G::M_BYTES;
       mbar_expect_tx(bar, m_bytes);
       if (need_m) tma_load_4d(smem_u32(dst), &maps.m, tx0, ty0, k, 0, bar);
-      if (need_t) tma_load_4d(smem_u32(dst + 9 * PLANE * 2), &maps.t, tx0, ty0, k, 0, bar);
+      if (need_t)
+        tma_load_4d(smem_u32(dst + 9 * PLANE * 2), tsel == kTsOld ? &maps.x : &maps.t, tx0, ty0, k,
+                    0, bar);
     };
     if (tid == 0) {
       for (int n = 0; n < NW - 1 && n < nplanes; ++n) issue_w(n);
       for (int o = 0; o < NC && o < nout; ++o) issue_c(o);
-      if (need_t)
+      if (ring_m)
         for (int o = 0; o < NM && o < nout; ++o) issue_m(o);
     }
 
@@ -1008,7 +1050,7 @@ __global__ void __launch_bounds__(256, 1)
       bool ok = mbar_wait_bounded(smem_u32(&bw[(fw0 + n) % NW]), ((fw0 + n) / NW) & 1);
       if (o >= 0) {
         ok = ok && mbar_wait_bounded(smem_u32(&bc[(fc0 + o) % NC]), ((fc0 + o) / NC) & 1);
-        if (need_t) ok = ok && mbar_wait_bounded(smem_u32(&bm[(fm0 + o) % NM]), ((fm0 + o) / NM) & 1);
+        if (ring_m) ok = ok && mbar_wait_bounded(smem_u32(&bm[(fm0 + o) % NM]), ((fm0 + o) / NM) & 1);
       }
       // Every thread waits on the ring barriers itself, so no block barrier is
       // needed before the plane is read; a thread whose wait expired skips the
@@ -1082,14 +1124,17 @@ __global__ void __launch_bounds__(256, 1)
           if (RK == 0) {
             base_t = base_o = win[v][P1];
           } else if (RK == 1) {
-            base_t = ld2(ts + v * PLANE + cidx);
+            base_t = need_t ? ld2(ts + v * PLANE + cidx) : pk(0.0f);
             base_o = ld2(ms + v * PLANE + cidx);
           } else {
             base_t = pk(0.0f);
             base_o = ld2(ts + v * PLANE + cidx);
           }
           st2(a.wout + q, f2fma(pk(cO), h[v], base_o));
-          if (RK <= 1) st2(a.t + q, f2fma(pk(cT), h[v], base_t));
+          if (RK == 0 ? !lean : RK == 1 && need_t)
+            st2(a.t + q, RK == 1 && tsel == kTsOld
+                             ? t_of_stages(base_o, base_t, win[v][P1], cT, h[v])
+                             : f2fma(pk(cT), h[v], base_t));
         }
       }
       __syncthreads();  // every thread is done with W plane n-1, C and M slot of o
@@ -1097,7 +1142,7 @@ __global__ void __launch_bounds__(256, 1)
       if (tid == 0) {
         if (n + NW - 1 < nplanes) issue_w(n + NW - 1);
         if (o >= 0 && o + NC < nout) issue_c(o + NC);
-        if (o >= 0 && need_t && o + NM < nout) issue_m(o + NM);
+        if (o >= 0 && ring_m && o + NM < nout) issue_m(o + NM);
       }
       return true;
     };
@@ -1122,7 +1167,7 @@ __global__ void __launch_bounds__(256, 1)
         const int o = n - 4 > 0 ? n - 4 : 0;
         for (int m = o; m < nout && m < o + NC; ++m)
           mbar_wait_bounded(smem_u32(&bc[(fc0 + m) % NC]), ((fc0 + m) / NC) & 1);
-        if (need_t)
+        if (ring_m)
           for (int m = o; m < nout && m < o + NM; ++m)
             mbar_wait_bounded(smem_u32(&bm[(fm0 + m) % NM]), ((fm0 + m) / NM) & 1);
       }
@@ -1130,7 +1175,7 @@ __global__ void __launch_bounds__(256, 1)
     }
     fw0 += nplanes;
     fc0 += nout;
-    if (need_t) fm0 += nout;
+    if (ring_m) fm0 += nout;
   }
 }
 
@@ -1410,7 +1455,7 @@ template <typename S> bool stage_stream_supported() { return true; }
 template <> bool stage_stream_supported<double>();
 template <>
 int encode_stream_maps<double>(const double *, const double *, const double *, const double *,
-                               const Layout &, void *);
+                               const double *, const Layout &, void *);
 template <>
 cudaError_t launch_stage_stream_batch<double>(const StageArgs<double> *, const void *const *, int,
                                               int *, int *, cudaStream_t, int *);
@@ -1419,8 +1464,8 @@ cudaError_t launch_stage_stream<double>(const StageArgs<double> &, const void *,
                                         cudaStream_t, cudaEvent_t, int *, int);
 
 template <typename S>
-int encode_stream_maps(const S *wave, const S *cjm, const S *wm, const S *t, const Layout &L,
-                       void *out) {
+int encode_stream_maps(const S *wave, const S *cjm, const S *wm, const S *t, const S *x,
+                       const Layout &L, void *out) {
   static_assert(sizeof(MapSet) <= kStreamMapsBytes, "tensor-map buffer too small");
   MapSet ms;
   int rc = CGFDM_OK;
@@ -1431,6 +1476,7 @@ int encode_stream_maps(const S *wave, const S *cjm, const S *wm, const S *t, con
     if (!rc) rc = encode_map<S>(cjm, L, 13, TX, ty, 3, &m.c3);
     if (!rc) rc = encode_map<S>(wm, L, 9, TX, ty, 9, &m.m);
     if (!rc) rc = encode_map<S>(t, L, 9, TX, ty, 9, &m.t);
+    if (!rc) rc = encode_map<S>(x, L, 9, TX, ty, 9, &m.x);
   }
   if constexpr (sizeof(S) == 2) {  // the paired-point kernel's 64 x 8 tiles
     using G = PairGeo<S>;
@@ -1440,6 +1486,7 @@ int encode_stream_maps(const S *wave, const S *cjm, const S *wm, const S *t, con
     if (!rc) rc = encode_map<S>(cjm, L, 13, G::TXP, G::TY, 3, &m.c3);
     if (!rc) rc = encode_map<S>(wm, L, 9, G::TXP, G::TY, 9, &m.m);
     if (!rc) rc = encode_map<S>(t, L, 9, G::TXP, G::TY, 9, &m.t);
+    if (!rc) rc = encode_map<S>(x, L, 9, G::TXP, G::TY, 9, &m.x);
   }
   if (!rc) std::memcpy(out, &ms, sizeof ms);
   return rc;

@@ -9,7 +9,8 @@ template cudaError_t launch_stage_stream_batch<__nv_bfloat16>(const StageArgs<__
 template bool stage_stream_supported<__nv_bfloat16>();
 template int encode_stream_maps<__nv_bfloat16>(const __nv_bfloat16 *, const __nv_bfloat16 *,
                                                const __nv_bfloat16 *, const __nv_bfloat16 *,
-                                               const Layout &, void *);
+                                               const __nv_bfloat16 *,
+                                        const Layout &, void *);
 template cudaError_t launch_stage_stream<__nv_bfloat16>(const StageArgs<__nv_bfloat16> &,
                                                         const void *, int *, int *, cudaStream_t, cudaEvent_t, int *, int);
 

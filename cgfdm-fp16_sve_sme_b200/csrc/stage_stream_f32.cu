@@ -8,7 +8,7 @@ template <> bool stage_stream_supported<double>() { return false; }
 
 template <>
 int encode_stream_maps<double>(const double *, const double *, const double *, const double *,
-                               const Layout &, void *) {
+                               const double *, const Layout &, void *) {
   set_error("no streaming kernel for FP64");
   return CGFDM_ERR_ARG;
 }
@@ -30,7 +30,7 @@ template cudaError_t launch_stage_stream_batch<float>(const StageArgs<float> *,
                                                       cudaStream_t, int *);
 template bool stage_stream_supported<float>();
 template int encode_stream_maps<float>(const float *, const float *, const float *, const float *,
-                                       const Layout &, void *);
+                                       const float *, const Layout &, void *);
 template cudaError_t launch_stage_stream<float>(const StageArgs<float> &, const void *, int *,
                                                 int *, cudaStream_t, cudaEvent_t, int *, int);
 

@@ -196,17 +196,23 @@ __global__ void __launch_bounds__(TTX *TTY) stage_top_kernel(const __grid_consta
       switch (a.irk) {
         case 0: {
           const float mv = ldv(W + q);
-          stv(a.t + q, mv + kB1 * h[v]);
+          if (!a.lean) stv(a.t + q, mv + kB1 * h[v]);
           stv(a.wout + q, mv + kA2rk * h[v]);
         } break;
         case 1:
-          stv(a.t + q, ldv(a.t + q) + kB2 * h[v]);
+          if (!a.lean) stv(a.t + q, ldv(a.t + q) + kB2 * h[v]);
           stv(a.wout + q, ldv(a.wm + q) + kA3rk * h[v]);
           break;
-        case 2:
-          stv(a.t + q, ldv(a.t + q) + kB3 * h[v]);
-          stv(a.wout + q, ldv(a.wm + q) + h[v]);
-          break;
+        case 2: {
+          const float mv = ldv(a.wm + q);
+          if (a.lean) {
+            const float w1 = ldv(a.wout + q), w2 = ldv(W + q);
+            stv(a.t + q, mv + (kT1 * (w1 - mv) + (kT2 * (w2 - mv) + kB3 * h[v])));
+          } else {
+            stv(a.t + q, ldv(a.t + q) + kB3 * h[v]);
+          }
+          stv(a.wout + q, mv + h[v]);
+        } break;
         default:
           stv(a.wout + q, ldv(a.t + q) + kB4 * h[v]);
       }
