@@ -13,8 +13,8 @@
 // four-buffer scheme per slab.
 //
 // Kernel choice per stage: the TMA-staged streaming kernel updates the
-// planes below the three free-surface layers and the exact-order kernel the
-// top three layers (KERNEL_STREAM / AUTO); KERNEL_EXACT runs the exact-order
+// planes below the three free-surface layers and the surface kernel those
+// (KERNEL_STREAM / AUTO); KERNEL_EXACT runs the exact-order
 // kernel everywhere (bit-identical to the reference's FP32 CPU build).
 #include <cuda_runtime.h>
 
@@ -74,7 +74,8 @@ std::map<std::tuple<int, int, int, int, int, int, int>, Tuned> g_tuned;
 // choice it times is written back.  The file is a JSON object whose members
 // map a key naming the GPU (name and SM count), the precision, the grid, the
 // PML width, a fixed work-item depth (or -1) and batch membership to
-// [tile form, work-item depth, tiled free-surface kernel 0/1].  A malformed
+// [tile form, work-item depth, tiled free-surface kernel 0/1] (the tuner
+// writes 1 there; 0 in a file selects the exact-order kernel).  A malformed
 // file or entry is ignored (the tuner times as if it were absent); writers
 // replace the file whole through a rename, so concurrent processes can lose
 // each other's new entries but never leave a partial file.  The load and
@@ -937,31 +938,10 @@ template <typename S> class EngineT : public Engine {
           best_chunk = ch;
         }
       }
-    // the free-surface layers: the tiled kernel (with the exact-order kernel
-    // on the PML-slab columns) against the exact-order kernel alone, on the
-    // surface of stage 0 (it writes X and T there, which stage 0 rewrites)
-    // (a batch member keeps its own choice, so that it computes the same
-    // bits alone and in the batch)
-    float surf_ms[2] = {0, 0};
-    for (int v = 0; v < 2 && err == cudaSuccess && !batch_form; ++v) {
-      fast_top_ = v == 0;
-      const StageArgs<S> s0 = stage_args(0, fb0, true);
-      const int l0 = launches_;
-      err = launch_surface(s0, st);
-      if (err == cudaSuccess) err = cudaEventRecord(e0, st);
-      for (int r = 0; r < 2 && err == cudaSuccess; ++r) err = launch_surface(s0, st);
-      if (err == cudaSuccess) err = cudaEventRecord(e1, st);
-      if (err == cudaSuccess) err = cudaEventSynchronize(e1);
-      if (err == cudaSuccess) err = cudaEventElapsedTime(&surf_ms[v], e0, e1);
-      launches_ = l0;
-    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     CUDA_TRY(err);
-    if (!batch_form) {
-      fast_top_ = surf_ms[0] <= surf_ms[1];
-      tile_rows_ = best_form;
-    }
+    if (!batch_form) tile_rows_ = best_form;
     chunk_ = best_chunk;
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tuned[key] = {best_form, best_chunk, fast_top_};
@@ -1002,7 +982,10 @@ template <typename S> class EngineT : public Engine {
       // read in 3)
       static const int nfield[4] = {30, 39, 57, 39};
       stream_bytes_ += (double)nfield[irk] * sizeof(S) * (double)(g_.nx) * g_.ny * (ksurf - HALO);
-      CUDA_TRY(launch_surface(a, st));
+      if (fast_top_)
+        CUDA_TRY(launch_surface(&a, 1, st));
+      else
+        CUDA_TRY(launch_surface_exact(a, st));
     } else {
       if (ev) {
         CUDA_TRY(cudaEventRecord(ev[1], st));
@@ -1020,35 +1003,29 @@ template <typename S> class EngineT : public Engine {
     return CGFDM_OK;
   }
 
-  // The three free-surface layers of a fast-path stage: the tiled kernel on
-  // the columns outside the PML slabs, the exact-order kernel on the slab
-  // columns (FP64 runs the exact-order kernel only).
-  cudaError_t launch_surface(const StageArgs<S> &a0, cudaStream_t st) {
-    StageArgs<S> a = a0;
-    a.kbeg = g_.L.nz_ - HALO - 3;
-    a.kend = g_.L.nz_ - HALO;
-    if constexpr (std::is_same<S, double>::value) {
-      ++launches_;
-      return launch_stage_exact<S>(a, st);
-    } else {
-      if (!fast_top_) {
-        ++launches_;
-        return launch_stage_exact<S>(a, st);
-      }
-      launches_ += g_.npml > 0 ? 2 : 1;
-      return launch_stage_top<S>(a, st);
-    }
+  // The three free-surface layers of a fast-path stage of n scenarios.
+  cudaError_t launch_surface(const StageArgs<S> *args, int n, cudaStream_t st) {
+    if constexpr (std::is_same<S, double>::value)
+      return cudaErrorNotSupported;  // FP64 runs the exact-order kernel only
+    else
+      return launch_stage_surface<S>(args, n, st, &launches_);
   }
 
-  // The free-surface layers of stage irk (the streaming part of the stage
-  // runs in a batch launch).
-  int launch_top(int irk, const int fb[3], cudaStream_t st) {
+  // The same by the exact-order kernel.
+  cudaError_t launch_surface_exact(StageArgs<S> a, cudaStream_t st) {
+    a.kbeg = g_.L.nz_ - HALO - 3;
+    a.kend = g_.L.nz_ - HALO;
+    ++launches_;
+    return launch_stage_exact<S>(a, st);
+  }
+
+  // The arguments of stage irk of a member whose launches the batch makes.
+  StageArgs<S> batch_stage(int irk, const int fb[3]) {
     static const int out_of[4] = {1, 2, 1, 0};
     StageArgs<S> a = stage_args(irk, fb, true);
     last_out_ = a.wout;
     last_aux_out_ = aux_total_ > 0 ? auxbuf(out_of[irk]) : nullptr;
-    CUDA_TRY(launch_surface(a, st));
-    return CGFDM_OK;
+    return a;
   }
 
   cudaError_t upload_repacked(const float *src, S *dst, int nfield) {
@@ -1159,8 +1136,8 @@ template <typename S> class EngineT : public Engine {
   int launches_ = 0;          // kernels launched by the last run()
   int tile_rows_ = 0;         // streaming-kernel tile height; 0 = autotune at the first run()
   int chunk_ = 0;             // planes per streaming work item in z; 0 = automatic
+  bool fast_top_ = true;      // free-surface layers on the tiled kernel (see Tuned)
   bool chunk_fixed_ = false;  // set by set_chunk: the autotuner keeps chunk_
-  bool fast_top_ = true;      // free-surface layers: tiled kernel + exact on slab columns
   bool drop_next_load_ = false;  // fault injection for failure-detection tests
   int *step_ = nullptr;       // device copy of it_, then the end-of-step kernel's block counter
   float *moment_tab_ = nullptr;            // point-source moment per step
@@ -1308,12 +1285,22 @@ template <typename S> class BatchT : public BatchBase {
           CUDA_TRY(launch_stage_stream_batch<S>(args.data(), maps.data(), (int)args.size(), err_,
                                                 err_ + 1, st));
       }
+      args.clear();
       for (auto *m : m_) {
         int fb[3];
         m->step_fb(irk, fb);
-        int rc = m->use_stream_ ? m->launch_top(irk, fb, st) : m->launch_stage(irk, fb, st, true);
-        if (rc) return rc;
+        if (m->use_stream_) {
+          const StageArgs<S> a = m->batch_stage(irk, fb);
+          if (m->fast_top_)
+            args.push_back(a);
+          else
+            CUDA_TRY(m->launch_surface_exact(a, st));
+        } else {
+          int rc = m->launch_stage(irk, fb, st, true);
+          if (rc) return rc;
+        }
       }
+      if (!args.empty()) CUDA_TRY(m_[0]->launch_surface(args.data(), (int)args.size(), st));
     }
     for (auto *m : m_) {
       int rc = m->step_end(st);

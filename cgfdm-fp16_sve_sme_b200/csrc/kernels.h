@@ -19,10 +19,13 @@ template <> struct SCALE_OF<__nv_bfloat16> { static constexpr double cv = 5.0e3,
 // Exact-order fused stage over the points kbeg <= k < kend (all i, j).
 template <typename S> cudaError_t launch_stage_exact(const StageArgs<S> &a, cudaStream_t st);
 
-// The three free-surface layers of the fast path: a shared-memory tiled
-// kernel for the columns outside every PML slab and the exact-order kernel
-// for the slab columns (FP32, FP16, BF16 storage).
-template <typename S> cudaError_t launch_stage_top(const StageArgs<S> &a, cudaStream_t st);
+// The three free-surface layers of one fast-path stage of n scenarios, all
+// columns, kSurfBatch scenarios per launch (FP32, FP16, BF16 storage).
+// `nlaunch` (optional) is increased by the number of kernels launched.
+constexpr int kSurfBatch = 16;
+template <typename S>
+cudaError_t launch_stage_surface(const StageArgs<S> *args, int n, cudaStream_t st,
+                                 int *nlaunch = nullptr);
 
 // TMA-staged z-streaming fused stage over kbeg <= k < kend, which must lie
 // below the three free-surface layers.  `maps` holds the tensor maps of the

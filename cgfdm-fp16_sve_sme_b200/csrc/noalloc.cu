@@ -168,7 +168,7 @@ int stage_noalloc(const cgfdm_stage_buffers &b, cudaStream_t st, unsigned char *
   if (overlap)
     NA_TRY(launch_stage_exact<S>(a, st));
   else  // the free-surface layers as a handle runs them
-    NA_TRY(launch_stage_top<S>(a, st));
+    NA_TRY(launch_stage_surface<S>(&a, 1, st));
   return CGFDM_OK;
 }
 

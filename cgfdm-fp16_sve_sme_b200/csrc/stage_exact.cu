@@ -79,6 +79,56 @@ template <typename R> __device__ __forceinline__ R LJT(const R *jt, int fb, R rD
   return fb > 0 ? LJT_fb<1>(jt, rDH) : LJT_fb<-1>(jt, rDH);
 }
 
+// What the RK combination of one value reads: the stage input `in`, `base`,
+// which the output adds the increment to (the step state m; in stage 3 the
+// accumulator t), and `acc`, which t adds it to (in stage 2 of a whole fast
+// step stage 1's input, still in the output buffer, see StageArgs::lean).
+template <typename S, typename A, typename R>
+__device__ __forceinline__ void rk_load(const StageArgs<S> &a, const A *win, const A *wm,
+                                        const A *t, const A *wout, long long q, R &in, R &base,
+                                        R &acc) {
+  in = acc = (R)0.0f;
+  switch (a.irk) {
+    case 0:
+      base = ldv(win + q);
+      break;
+    case 1:
+      base = ldv(wm + q);
+      if (!a.lean) acc = ldv(t + q);
+      break;
+    case 2:
+      base = ldv(wm + q);
+      acc = ldv((a.lean ? wout : t) + q);
+      if (a.lean) in = ldv(win + q);
+      break;
+    default:
+      base = ldv(t + q);
+  }
+}
+// The new accumulator t (stages 0-2) and output o of one value.
+template <typename S, typename R>
+__device__ __forceinline__ void rk_apply(const StageArgs<S> &a, R in, R base, R acc, R h, R &t,
+                                         R &o) {
+  t = (R)0.0f;
+  switch (a.irk) {
+    case 0:
+      t = base + (R)kB1 * h;
+      o = base + (R)kA2rk * h;
+      break;
+    case 1:
+      t = acc + (R)kB2 * h;
+      o = base + (R)kA3rk * h;
+      break;
+    case 2:
+      t = a.lean ? base + ((R)kT1 * (acc - base) + ((R)kT2 * (in - base) + (R)kB3 * h))
+                 : acc + (R)kB3 * h;
+      o = base + h;
+      break;
+    default:
+      o = base + (R)kB4 * h;
+  }
+}
+
 template <typename S>
 __global__ void __launch_bounds__(256) stage_exact_kernel(StageArgs<S> a) {
   using R = typename Arith<S>::R;
@@ -87,7 +137,6 @@ __global__ void __launch_bounds__(256) stage_exact_kernel(StageArgs<S> a) {
   const int k = blockIdx.z * blockDim.z + threadIdx.z + a.kbeg;
   const int nx_ = a.L.nx_, ny_ = a.L.ny_, nz_ = a.L.nz_;
   if (i >= nx_ - HALO || j >= ny_ - HALO || k >= a.kend) return;
-  if (i >= a.skip_i0 && i < a.skip_i1 && j >= a.skip_j0 && j < a.skip_j1) return;
   const long long num = a.L.fs;  // field stride
   const long long sx = 1, sy = a.L.px, sz = a.L.plane;
   const long long c = a.L.at(i, j, k);
@@ -237,66 +286,35 @@ __global__ void __launch_bounds__(256) stage_exact_kernel(StageArgs<S> a) {
 #pragma unroll
       for (int v = 3; v < 9; ++v) ha[v] = ha[v] + t[v] * DT;
     }
-    // pml_rk.cpp:15-69
+    // pml_rk.cpp:15-69.  All nine values are loaded before the first store: a
+    // load behind a store that may alias it waits for it, which made the
+    // updates of stages 1-3 chains of nine memory round trips.
     R *aout = sl.aout + pos;
     R *at = sl.at + pos;
     const R *am = sl.am + pos;
+    R base[9], acc[9], in[9];
+#pragma unroll
+    for (int v = 0; v < 9; ++v) rk_load(a, ain, am, at, aout, v * np, in[v], base[v], acc[v]);
 #pragma unroll
     for (int v = 0; v < 9; ++v) {
-      const R hv = ha[v];
-      const long long q = v * np;
-      switch (a.irk) {
-        case 0: {
-          const R mv = ain[q];
-          if (!a.lean) at[q] = mv + (R)kB1 * hv;
-          aout[q] = mv + (R)kA2rk * hv;
-        } break;
-        case 1:
-          if (!a.lean) at[q] = at[q] + (R)kB2 * hv;
-          aout[q] = am[q] + (R)kA3rk * hv;
-          break;
-        case 2: {
-          const R mv = am[q];
-          at[q] = a.lean ? mv + ((R)kT1 * (aout[q] - mv) + ((R)kT2 * (ain[q] - mv) + (R)kB3 * hv))
-                         : at[q] + (R)kB3 * hv;
-          aout[q] = mv + hv;
-        } break;
-        default:
-          aout[q] = at[q] + (R)kB4 * hv;
-      }
+      R t, o;
+      rk_apply(a, in[v], base[v], acc[v], ha[v], t, o);
+      if (a.irk < 3 && (!a.lean || a.irk == 2)) at[v * np] = t;
+      aout[v * np] = o;
     }
   }
 
-  // wave_rk.cpp:13-99
+  // wave_rk.cpp:13-99, loads before stores as above
+  {
+    R base[9], acc[9], in[9];
 #pragma unroll
-  for (int v = 0; v < 9; ++v) {
-    const long long q = c + v * num;
-    const R hv = h[v];
-    switch (a.irk) {
-      case 0: {
-        const R mv = ldv(W + q);
-        if (!a.lean) stv(a.t + q, mv + (R)kB1 * hv);
-        stv(a.wout + q, mv + (R)kA2rk * hv);
-      } break;
-      case 1: {
-        const R mv = ldv(a.wm + q);
-        if (!a.lean) stv(a.t + q, (R)ldv(a.t + q) + (R)kB2 * hv);
-        stv(a.wout + q, mv + (R)kA3rk * hv);
-      } break;
-      case 2: {
-        const R mv = ldv(a.wm + q);
-        if (a.lean) {
-          const R w1 = ldv(a.wout + q), w2 = ldv(W + q);
-          stv(a.t + q, mv + ((R)kT1 * (w1 - mv) + ((R)kT2 * (w2 - mv) + (R)kB3 * hv)));
-        } else {
-          stv(a.t + q, (R)ldv(a.t + q) + (R)kB3 * hv);
-        }
-        stv(a.wout + q, mv + hv);
-      } break;
-      default: {
-        const R tv = ldv(a.t + q);
-        stv(a.wout + q, tv + (R)kB4 * hv);
-      }
+    for (int v = 0; v < 9; ++v) rk_load(a, W, a.wm, a.t, a.wout, c + v * num, in[v], base[v], acc[v]);
+#pragma unroll
+    for (int v = 0; v < 9; ++v) {
+      R t, o;
+      rk_apply(a, in[v], base[v], acc[v], h[v], t, o);
+      if (a.irk < 3 && (!a.lean || a.irk == 2)) stv(a.t + c + v * num, t);
+      stv(a.wout + c + v * num, o);
     }
   }
 }

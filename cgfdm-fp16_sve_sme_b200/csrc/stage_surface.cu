@@ -16,6 +16,10 @@
 // m, t and the auxiliaries, each behind a store that might alias it, took one
 // round trip per field.  Hence one layer per block, every load of a phase
 // issued before its first store, and no second launch for the slab columns.
+// Measured per stage against the two launches before (three layers per block,
+// the exact-order kernel on the slab columns): 64x64x48 40-80 -> 13.5 us,
+// 401x401x201 with a 20-cell PML 90-168 -> 61-72 us, 601x601x401 145-263 ->
+// 125-149 us (FP32, cold cache).
 // FP32 arithmetic with FMA contraction, equal to the reference up to rounding.
 #include <algorithm>
 
