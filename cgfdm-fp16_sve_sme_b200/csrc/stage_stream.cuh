@@ -217,6 +217,17 @@ __device__ __forceinline__ float stencil1(float t0, float t1, float t2, float t3
   return fmaf(kA3, t4, fmaf(kA2, t3, fmaf(kA1, t2, fmaf(kA0, t1, kAm1 * t0))));
 }
 
+// Stage classes RK of the kernels: 0, 1 (stages 1 and 2) and 3 update the
+// accumulator as the reference does; 4, 5 and 6 are stages 0, 1 and 2 of a
+// whole step (StageArgs::lean), whose stage 3 is class 3 too.  Compile-time
+// classes: with the form chosen at run time the PML variant of stages 1-2
+// spilled 28-60 bytes a thread at its 128 registers.
+enum { kTsAcc = 0, kTsNone = 1, kTsOld = 2 };  // what t comes from, if it is written
+template <int RK> constexpr int stage_of() { return RK == 4 ? 0 : RK >= 5 ? 1 : RK; }
+template <int RK> constexpr int tsel_of() {
+  return RK == 4 || RK == 5 ? kTsNone : RK == 6 ? kTsOld : kTsAcc;
+}
+
 // t from the step state m, the inputs w1 and w2 of stages 1 and 2 and stage
 // 2's increment h (see StageArgs::lean).
 __device__ __forceinline__ float2 t_of_stages(float2 m, float2 w1, float2 w2, float cB, float2 h) {
@@ -239,76 +250,75 @@ __device__ __forceinline__ unsigned slab_pos(const SlabDev<float> &sl, int i, in
 //
 // A point's inputs are the auxiliary input (part 1), what the stage adds the
 // increment to (part 2: m in stages 1-2, t in stage 3) and what t comes from
-// (part 4, stages 1-2; tsel: kTsAcc = t itself, kTsNone = no t in this stage,
-// kTsOld = stage 1's input, which the output buffer still holds, see
+// (part 4, stages 1-2; tsel_of: kTsAcc = t itself, kTsNone = no t in this
+// stage, kTsOld = stage 1's input, which the output buffer still holds, see
 // StageArgs::lean).  pml_load<RK> loads the parts in a mask for all nine fields, so that
 // the loads can be issued at the top of a plane iteration and their latency
 // overlaps the stencil work; pml_apply<RK> is told which parts are already
 // in registers (a compile-time or a per-thread mask), loads the others
 // (three fields at a time, each group's loads before its stores) and updates.
-template <int RK> constexpr int pml_parts() { return RK == 0 ? 1 : RK == 3 ? 3 : 7; }
+template <int RK> constexpr int pml_parts() {
+  return stage_of<RK>() == 0 ? 1 : tsel_of<RK>() == kTsNone || RK == 3 ? 3 : 7;
+}
 struct PmlIn {
   float a[9], b[9], t[9];
 };
-enum { kTsAcc = 0, kTsNone = 1, kTsOld = 2 };
 template <int RK>
 __device__ __forceinline__ void pml_load_fields(const SlabDev<float> &sl, unsigned pos, int v0,
-                                                int nv, int mask, int tsel, PmlIn &in) {
+                                                int nv, int mask, PmlIn &in) {
   constexpr int P = pml_parts<RK>();
   const unsigned np = (unsigned)sl.np;
-  const float *tp = tsel == kTsOld ? sl.aout : sl.at;
+  const float *tp = tsel_of<RK>() == kTsOld ? sl.aout : sl.at;
 #pragma unroll
   for (int v = v0; v < v0 + nv; ++v) {
     const unsigned q = v * np + pos;
     if ((P & 1) && (mask & 1)) in.a[v] = sl.ain[q];
     if ((P & 2) && (mask & 2)) in.b[v] = RK == 3 ? sl.at[q] : sl.am[q];
-    if ((P & 4) && (mask & 4) && tsel != kTsNone) in.t[v] = tp[q];
+    if ((P & 4) && (mask & 4)) in.t[v] = tp[q];
   }
 }
 template <int RK>
-__device__ __forceinline__ void pml_load(const SlabDev<float> &sl, unsigned pos, int mask, int tsel,
-                                         PmlIn &in) {
-  pml_load_fields<RK>(sl, pos, 0, 9, mask, tsel, in);
+__device__ __forceinline__ void pml_load(const SlabDev<float> &sl, unsigned pos, int mask, PmlIn &in) {
+  pml_load_fields<RK>(sl, pos, 0, 9, mask, in);
 }
 // L1 prefetch of the parts in a mask (no registers held), for the parts the
 // stage needs but does not keep in registers across the stencils.
 template <int RK>
-__device__ __forceinline__ void pml_prefetch(const SlabDev<float> &sl, unsigned pos, int mask,
-                                             int tsel) {
+__device__ __forceinline__ void pml_prefetch(const SlabDev<float> &sl, unsigned pos, int mask) {
   constexpr int P = pml_parts<RK>();
   const unsigned np = (unsigned)sl.np;
-  const float *tp = tsel == kTsOld ? sl.aout : sl.at;
+  const float *tp = tsel_of<RK>() == kTsOld ? sl.aout : sl.at;
 #pragma unroll
   for (int v = 0; v < 9; ++v) {
     const unsigned q = v * np + pos;
     if ((P & 2) && (mask & 2))
       asm volatile("prefetch.global.L1 [%0];" ::"l"(RK == 3 ? sl.at + q : sl.am + q));
-    if ((P & 4) && (mask & 4) && tsel != kTsNone)
+    if ((P & 4) && (mask & 4))
       asm volatile("prefetch.global.L1 [%0];" ::"l"(tp + q));
   }
 }
 template <int RK>
 __device__ __forceinline__ void pml_apply(const SlabDev<float> &sl, unsigned pos, const float E[9],
                                           float dl, float ad, float bt, float DT, float cB,
-                                          float cA, float h[9], int held, int tsel, int lean,
-                                          PmlIn &in) {
+                                          float cA, float h[9], int held, PmlIn &in) {
+  constexpr int ST = stage_of<RK>(), tsel = tsel_of<RK>();
   const unsigned np = (unsigned)sl.np;
   // (not __restrict__: with kTsOld part 4 is read through aout as well)
   float *aout = sl.aout;
   float *at = sl.at;
 #pragma unroll
   for (int g = 0; g < 9; g += 3) {
-    pml_load_fields<RK>(sl, pos, g, 3, 7 & ~held, tsel, in);
+    pml_load_fields<RK>(sl, pos, g, 3, 7 & ~held, in);
 #pragma unroll
     for (int v = g; v < g + 3; ++v) {
       const unsigned q = v * np + pos;
       const float a = in.a[v];
       const float ha = (dl * E[v] - ad * a) * DT;
       h[v] -= bt * a * DT;
-      if (RK == 0) {
-        if (!lean) at[q] = a + kB1 * ha;
+      if (ST == 0) {
+        if (tsel == kTsAcc) at[q] = a + kB1 * ha;
         aout[q] = a + kA2rk * ha;
-      } else if (RK == 1) {
+      } else if (ST == 1) {
         const float m = in.b[v];
         if (tsel == kTsAcc) at[q] = in.t[v] + cB * ha;
         if (tsel == kTsOld) at[q] = m + (kT1 * (in.t[v] - m) + (kT2 * (a - m) + cB * ha));
@@ -320,11 +330,11 @@ __device__ __forceinline__ void pml_apply(const SlabDev<float> &sl, unsigned pos
   }
 }
 // The parts of a slab point loaded at the top of its plane iteration: all of
-// them in stages 0 and 3; the auxiliary input alone in stages 1-2, where
-// holding all three parts (27 registers) across the stencils spills.  The
+// them where there are at most two; the auxiliary input alone where holding
+// all three (27 registers) across the stencils spills.  The
 // loads are for the point's first slab in application order (x, then y,
 // then the bottom z slab); a corner point loads its later slabs in place.
-template <int RK> constexpr int hoist_parts() { return RK == 1 ? 1 : pml_parts<RK>(); }
+template <int RK> constexpr int hoist_parts() { return pml_parts<RK>() == 7 ? 1 : pml_parts<RK>(); }
 
 struct Maps {
   CUtensorMap w;   // stage input wavefield, box BX x BY x 1 x 9
@@ -487,13 +497,12 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
     const Maps &maps = src.maps(e);
     const Work &wk = src.work(e);
     const Layout L = a.L;
-    // stages 1 and 2 (RK = 1) differ in the weights of the t and output
-    // updates and, in a whole step (a.lean), in what t comes from
-    constexpr bool ring_m = RK >= 1, need_m = RK == 1;
-    const int lean = a.lean;
-    const int tsel = RK != 1 || !lean ? kTsAcc : a.irk == 2 ? kTsOld : kTsNone;
-    const bool need_t = RK >= 1 && tsel != kTsNone;
-    const float cB = a.irk == 2 ? kB3 : kB2, cA = a.irk == 2 ? 1.0f : kA3rk;
+    // stages 1 and 2 differ in the weights of the t and output updates and,
+    // in a whole step, in what t comes from
+    constexpr int ST = stage_of<RK>(), tsel = tsel_of<RK>();
+    constexpr bool ring_m = ST >= 1, need_m = ST == 1, need_t = ST >= 1 && tsel != kTsNone;
+    const bool second = RK == 6 || (RK == 1 && a.irk == 2);
+    const float cB = second ? kB3 : kB2, cA = second ? 1.0f : kA3rk;
     const uint32_t m_bytes = (need_m ? 9 : 0) * NTHR * G::ES + (need_t ? 9 : 0) * NTHR * G::ES;
     const float rDH = a.rDH, DT = a.DT;
     // the MacCormack sign and 1/DH of each direction, applied to its elastic
@@ -602,9 +611,9 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
         sh = sx >= 0 ? sx : sy >= 0 ? sy : kk < HALO + a.npml ? 2 : -1;
         if (sh >= 0) {
           const unsigned pos = slab_pos(a.slab[sh], i, j, kk);
-          pml_load<RK>(a.slab[sh], pos, HP, tsel, pin);
+          pml_load<RK>(a.slab[sh], pos, HP, pin);
           if (HP != pml_parts<RK>())
-            pml_prefetch<RK>(a.slab[sh], pos, pml_parts<RK>() & ~HP, tsel);
+            pml_prefetch<RK>(a.slab[sh], pos, pml_parts<RK>() & ~HP);
         }
       }
       bool ok = mbar_wait_bounded(smem_u32(&bw[(fw0 + n) % NW]), ((fw0 + n) / NW) & 1);
@@ -685,8 +694,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
         if constexpr (PMLK) {
           if (sx >= 0) {  // profile values d, alpha + d, beta at this x
             elastic9(mx, Lr, mu, lam, bu, E);
-            pml_apply<RK>(a.slab[sx], slab_pos(a.slab[sx], i, j, k), E, dlx, adx, btx, DT, cB, cA, pc, HP, tsel,
-                          lean, pin);
+            pml_apply<RK>(a.slab[sx], slab_pos(a.slab[sx], i, j, k), E, dlx, adx, btx, DT, cB, cA, pc, HP, pin);
           }
         }
         // y direction
@@ -710,7 +718,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
           if (sy >= 0) {
             elastic9(my, Lr, mu, lam, bu, E);
             pml_apply<RK>(a.slab[sy], slab_pos(a.slab[sy], i, j, k), E, dly, ady, bty, DT, cB, cA, pc,
-                          sh == sy ? HP : 0, tsel, lean, pin);
+                          sh == sy ? HP : 0, pin);
           }
         }
         // z direction: W[k - m*DIR] for m = -1..3 sits in slots P0 (q = k + DIR) .. P4
@@ -730,7 +738,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
             elastic9(mz, Lr, mu, lam, bu, E);
             const float d = __ldg(pz + 2 * L.nz_ + k), btz = __ldg(pz + L.nz_ + k), adz = __ldg(pz + k) + d;
             pml_apply<RK>(a.slab[2], slab_pos(a.slab[2], i, j, k), E, d * gz, adz, btz, DT, cB, cA, pc,
-                          sh == 2 ? HP : 0, tsel, lean, pin);
+                          sh == 2 ? HP : 0, pin);
           }
         }
         es.finish(mu, lam, bu, h);
@@ -747,8 +755,8 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
         const S *ms = (const S *)(smem + G::OFF_M + ((fm0 + o) % NM) * G::M_BYTES);
         const S *ts = ms + 9 * NTHR;
         const long long ctr = L.at(i, j, k);
-        const float cT = RK == 0 ? kB1 : RK == 1 ? cB : 0.0f;
-        const float cO = RK == 0 ? kA2rk : RK == 1 ? cA : kB4;
+        const float cT = ST == 0 ? kB1 : ST == 1 ? cB : 0.0f;
+        const float cO = ST == 0 ? kA2rk : ST == 1 ? cA : kB4;
 #pragma unroll
         for (int v = 0; v < 9; v += 2) {
           const bool two = v < 8;
@@ -756,9 +764,9 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
           const long long q = ctr + v * fs;
           float2 base_t, base_o;  // what t and the output add the increment to
           base_t = pk(0.0f);
-          if (RK == 0) {
+          if (ST == 0) {
             base_t = base_o = pk(win[v][P1], two ? win[v + 1][P1] : 0.0f);
-          } else if (RK == 1) {
+          } else if (ST == 1) {
             if (need_t)
               base_t = pk(ldv(ts + v * NTHR + cidx), two ? ldv(ts + (v + 1) * NTHR + cidx) : 0.0f);
             base_o = pk(ldv(ms + v * NTHR + cidx), two ? ldv(ms + (v + 1) * NTHR + cidx) : 0.0f);
@@ -768,9 +776,9 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
           const float2 wo = __ffma2_rn(pk(cO), hv, base_o);
           stv(a.wout + q, wo.x);
           if (two) stv(a.wout + q + fs, wo.y);
-          if (RK == 0 ? !lean : RK == 1 && need_t) {
+          if (ST <= 1 && tsel != kTsNone) {
             const float2 wt =
-                RK == 1 && tsel == kTsOld
+                tsel == kTsOld
                     ? t_of_stages(base_o, base_t, pk(win[v][P1], two ? win[v + 1][P1] : 0.0f), cT, hv)
                     : __ffma2_rn(pk(cT), hv, base_t);
             stv(a.t + q, wt.x);
@@ -966,11 +974,10 @@ __global__ void __launch_bounds__(256, 1)
 
   unsigned fw0 = 0, fc0 = 0, fm0 = 0;  // ring fill counters, continued across items
   const Layout L = a.L;
-  constexpr bool ring_m = RK >= 1, need_m = RK == 1;
-  const int lean = a.lean;  // see StageArgs::lean and the one-point kernel
-  const int tsel = RK != 1 || !lean ? kTsAcc : a.irk == 2 ? kTsOld : kTsNone;
-  const bool need_t = RK >= 1 && tsel != kTsNone;
-  const float cB = a.irk == 2 ? kB3 : kB2, cA = a.irk == 2 ? 1.0f : kA3rk;
+  constexpr int ST = stage_of<RK>(), tsel = tsel_of<RK>();
+  constexpr bool ring_m = ST >= 1, need_m = ST == 1, need_t = ST >= 1 && tsel != kTsNone;
+  const bool second = RK == 6 || (RK == 1 && a.irk == 2);
+  const float cB = second ? kB3 : kB2, cA = second ? 1.0f : kA3rk;
   const uint32_t m_bytes = ((need_m ? 9 : 0) + (need_t ? 9 : 0)) * PLANE * 2;
   const float rDH = a.rDH, DT = a.DT;
   const float gx = FB1 * rDH, gy = FB2 * rDH, gz = FB3 * rDH;
@@ -1115,15 +1122,15 @@ __global__ void __launch_bounds__(256, 1)
         const S *ms = (const S *)(smem + G::OFF_M + ((fm0 + o) % NM) * G::M_BYTES);
         const S *ts = ms + 9 * PLANE;
         const long long ctr = L.at(i, j, k);
-        const float cT = RK == 0 ? kB1 : RK == 1 ? cB : 0.0f;
-        const float cO = RK == 0 ? kA2rk : RK == 1 ? cA : kB4;
+        const float cT = ST == 0 ? kB1 : ST == 1 ? cB : 0.0f;
+        const float cO = ST == 0 ? kA2rk : ST == 1 ? cA : kB4;
 #pragma unroll
         for (int v = 0; v < 9; ++v) {
           const long long q = ctr + v * fs;
           float2 base_t, base_o;
-          if (RK == 0) {
+          if (ST == 0) {
             base_t = base_o = win[v][P1];
-          } else if (RK == 1) {
+          } else if (ST == 1) {
             base_t = need_t ? ld2(ts + v * PLANE + cidx) : pk(0.0f);
             base_o = ld2(ms + v * PLANE + cidx);
           } else {
@@ -1131,8 +1138,8 @@ __global__ void __launch_bounds__(256, 1)
             base_o = ld2(ts + v * PLANE + cidx);
           }
           st2(a.wout + q, f2fma(pk(cO), h[v], base_o));
-          if (RK == 0 ? !lean : RK == 1 && need_t)
-            st2(a.t + q, RK == 1 && tsel == kTsOld
+          if (ST <= 1 && tsel != kTsNone)
+            st2(a.t + q, tsel == kTsOld
                              ? t_of_stages(base_o, base_t, win[v][P1], cT, h[v])
                              : f2fma(pk(cT), h[v], base_t));
         }
@@ -1492,8 +1499,10 @@ int encode_stream_maps(const S *wave, const S *cjm, const S *wm, const S *t, con
   return rc;
 }
 
-// The stage class RK of stage irk: 0, 1 (stages 1 and 2) or 3.
-inline int rk_class(int irk) { return irk == 0 ? 0 : irk == 3 ? 3 : 1; }
+// The stage class of stage irk (see stage_of).
+inline int rk_class(int irk, int lean) {
+  return irk == 3 ? 3 : lean ? 4 + irk : irk == 0 ? 0 : 1;
+}
 
 template <typename S, int TYv, int RK>
 cudaError_t launch_fb_rk(const StageArgs<S> &a, const Maps &m, int *err, int *counter,
@@ -1525,26 +1534,20 @@ cudaError_t launch_fb_rk_pair(const StageArgs<S> &a, const MapSet &ms, int *err,
     default: return launch_one_pair<S, 1, 1, 1, RK>(a, m8, mp, err, counter, st, nlaunch);
   }
 }
-template <typename S>
-cudaError_t launch_pair(const StageArgs<S> &a, const MapSet &ms, int *err, int *counter,
-                        cudaStream_t st, int *nlaunch) {
-  switch (rk_class(a.irk)) {
-    case 0: return launch_fb_rk_pair<S, 0>(a, ms, err, counter, st, nlaunch);
-    case 1: return launch_fb_rk_pair<S, 1>(a, ms, err, counter, st, nlaunch);
-    default: return launch_fb_rk_pair<S, 3>(a, ms, err, counter, st, nlaunch);
+// One stage class of one scenario at the tile forms other than 32 x 16, and
+// of a batch at 32 x 16; instantiated in several translation units per
+// storage type, STREAM_PART of them (the classes of a part are listed at
+// STREAM_INSTANTIATE).
+template <typename S, int RK>
+cudaError_t launch_single_rk(const StageArgs<S> &a, const void *maps, int *err, int *counter,
+                             cudaStream_t st, int *nlaunch, int tile_rows) {
+  const MapSet &ms = *(const MapSet *)maps;
+  if (tile_rows == 8) return launch_fb_rk<S, 8, RK>(a, ms.ty8, err, counter, st, nlaunch);
+  if constexpr (sizeof(S) == 2) {
+    if (tile_rows == kTilePair) return launch_fb_rk_pair<S, RK>(a, ms, err, counter, st, nlaunch);
   }
+  return cudaErrorInvalidValue;
 }
-
-template <typename S, int TYv>
-cudaError_t launch_fb(const StageArgs<S> &a, const Maps &m, int *err, int *counter,
-                      cudaStream_t st, int *nlaunch) {
-  switch (rk_class(a.irk)) {
-    case 0: return launch_fb_rk<S, TYv, 0>(a, m, err, counter, st, nlaunch);
-    case 1: return launch_fb_rk<S, TYv, 1>(a, m, err, counter, st, nlaunch);
-    default: return launch_fb_rk<S, TYv, 3>(a, m, err, counter, st, nlaunch);
-  }
-}
-
 template <typename S, int RK>
 cudaError_t launch_batch_rk(const StageArgs<S> *args, const void *const *maps, int n, int *err,
                             int *counter, cudaStream_t st, int *nlaunch) {
@@ -1561,23 +1564,43 @@ cudaError_t launch_batch_rk(const StageArgs<S> *args, const void *const *maps, i
   }
 }
 
+#define STREAM_CLASS(EXT, S, RK)                                                                  \
+  EXT template cudaError_t launch_single_rk<S, RK>(const StageArgs<S> &, const void *, int *,     \
+                                                   int *, cudaStream_t, int *, int);              \
+  EXT template cudaError_t launch_batch_rk<S, RK>(const StageArgs<S> *, const void *const *, int, \
+                                                  int *, int *, cudaStream_t, int *);
+// The classes of a storage type over three translation units: part 0 the
+// single-stage forms and the dispatch, parts 1 and 2 whole steps.
+#if STREAM_PART == 0
+#define STREAM_INSTANTIATE(S)                                                            \
+  STREAM_CLASS(, S, 0) STREAM_CLASS(, S, 1)                                              \
+  STREAM_CLASS(extern, S, 3) STREAM_CLASS(extern, S, 4) STREAM_CLASS(extern, S, 5)       \
+  STREAM_CLASS(extern, S, 6)
+#elif STREAM_PART == 1
+#define STREAM_INSTANTIATE(S) STREAM_CLASS(, S, 3) STREAM_CLASS(, S, 4)
+#else
+#define STREAM_INSTANTIATE(S) STREAM_CLASS(, S, 5) STREAM_CLASS(, S, 6)
+#endif
+
 template <typename S>
 cudaError_t launch_stage_stream(const StageArgs<S> &a, const void *maps_in, int *err, int *counter,
                                 cudaStream_t st, cudaEvent_t after_main, int *nlaunch,
                                 int tile_rows) {
   if (a.kend <= a.kbeg) return cudaSuccess;
-  const MapSet &ms = *(const MapSet *)maps_in;
   // tile height 16 runs the batched kernel as a batch of one, so that a
   // scenario gives the same bits alone and inside a batch
   cudaError_t e;
-  if (tile_rows == kTilePair) {
-    if constexpr (sizeof(S) == 2)
-      e = launch_pair<S>(a, ms, err, counter, st, nlaunch);
-    else
-      e = cudaErrorInvalidValue;
+  if (tile_rows == 16) {
+    e = launch_stage_stream_batch<S>(&a, &maps_in, 1, err, counter, st, nlaunch);
   } else {
-    e = tile_rows == 8 ? launch_fb<S, 8>(a, ms.ty8, err, counter, st, nlaunch)
-                       : launch_stage_stream_batch<S>(&a, &maps_in, 1, err, counter, st, nlaunch);
+    switch (rk_class(a.irk, a.lean)) {
+      case 0: e = launch_single_rk<S, 0>(a, maps_in, err, counter, st, nlaunch, tile_rows); break;
+      case 1: e = launch_single_rk<S, 1>(a, maps_in, err, counter, st, nlaunch, tile_rows); break;
+      case 3: e = launch_single_rk<S, 3>(a, maps_in, err, counter, st, nlaunch, tile_rows); break;
+      case 4: e = launch_single_rk<S, 4>(a, maps_in, err, counter, st, nlaunch, tile_rows); break;
+      case 5: e = launch_single_rk<S, 5>(a, maps_in, err, counter, st, nlaunch, tile_rows); break;
+      default: e = launch_single_rk<S, 6>(a, maps_in, err, counter, st, nlaunch, tile_rows);
+    }
   }
   if (e != cudaSuccess) return e;
   if (after_main) e = cudaEventRecord(after_main, st);
@@ -1589,12 +1612,15 @@ cudaError_t launch_stage_stream_batch(const StageArgs<S> *args, const void *cons
   if (n <= 0) return cudaSuccess;
   for (int q = 1; q < n; ++q)
     if (args[q].fb1 != args[0].fb1 || args[q].fb2 != args[0].fb2 || args[q].fb3 != args[0].fb3 ||
-        args[q].irk != args[0].irk)
+        args[q].irk != args[0].irk || args[q].lean != args[0].lean)
       return cudaErrorInvalidValue;
-  switch (rk_class(args[0].irk)) {
+  switch (rk_class(args[0].irk, args[0].lean)) {
     case 0: return launch_batch_rk<S, 0>(args, maps, n, err, counter, st, nlaunch);
     case 1: return launch_batch_rk<S, 1>(args, maps, n, err, counter, st, nlaunch);
-    default: return launch_batch_rk<S, 3>(args, maps, n, err, counter, st, nlaunch);
+    case 3: return launch_batch_rk<S, 3>(args, maps, n, err, counter, st, nlaunch);
+    case 4: return launch_batch_rk<S, 4>(args, maps, n, err, counter, st, nlaunch);
+    case 5: return launch_batch_rk<S, 5>(args, maps, n, err, counter, st, nlaunch);
+    default: return launch_batch_rk<S, 6>(args, maps, n, err, counter, st, nlaunch);
   }
 }
 

@@ -3,6 +3,10 @@
 
 namespace cgfdm {
 
+STREAM_INSTANTIATE(__nv_bfloat16)
+
+#if STREAM_PART == 0
+
 template cudaError_t launch_stage_stream_batch<__nv_bfloat16>(const StageArgs<__nv_bfloat16> *,
                                                               const void *const *, int, int *,
                                                               int *, cudaStream_t, int *);
@@ -13,5 +17,7 @@ template int encode_stream_maps<__nv_bfloat16>(const __nv_bfloat16 *, const __nv
                                         const Layout &, void *);
 template cudaError_t launch_stage_stream<__nv_bfloat16>(const StageArgs<__nv_bfloat16> &,
                                                         const void *, int *, int *, cudaStream_t, cudaEvent_t, int *, int);
+
+#endif
 
 }  // namespace cgfdm

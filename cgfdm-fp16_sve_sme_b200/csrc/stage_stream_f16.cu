@@ -3,6 +3,10 @@
 
 namespace cgfdm {
 
+STREAM_INSTANTIATE(__half)
+
+#if STREAM_PART == 0
+
 template cudaError_t launch_stage_stream_batch<__half>(const StageArgs<__half> *,
                                                        const void *const *, int, int *, int *,
                                                        cudaStream_t, int *);
@@ -12,5 +16,7 @@ template int encode_stream_maps<__half>(const __half *, const __half *, const __
                                         const Layout &, void *);
 template cudaError_t launch_stage_stream<__half>(const StageArgs<__half> &, const void *, int *,
                                                  int *, cudaStream_t, cudaEvent_t, int *, int);
+
+#endif
 
 }  // namespace cgfdm

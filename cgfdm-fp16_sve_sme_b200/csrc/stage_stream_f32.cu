@@ -3,6 +3,10 @@
 
 namespace cgfdm {
 
+STREAM_INSTANTIATE(float)
+
+#if STREAM_PART == 0
+
 // FP64 has no streaming kernel (the exact-order kernel runs it)
 template <> bool stage_stream_supported<double>() { return false; }
 
@@ -33,5 +37,7 @@ template int encode_stream_maps<float>(const float *, const float *, const float
                                        const float *, const Layout &, void *);
 template cudaError_t launch_stage_stream<float>(const StageArgs<float> &, const void *, int *,
                                                 int *, cudaStream_t, cudaEvent_t, int *, int);
+
+#endif
 
 }  // namespace cgfdm
