@@ -178,6 +178,50 @@ Dims make_dims(const cgfdm_desc &d) {
 
 template <typename S> class BatchT;
 
+// Two side streams that branch off a caller's stream and join it again, for
+// the launches of one stage (its owner's host thread drives them).  Under
+// stream capture they become parallel branches of the graph.
+class Fork {
+ public:
+  cudaError_t create() {
+    cudaError_t e = cudaEventCreateWithFlags(&start_, cudaEventDisableTiming);
+    for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
+      e = cudaStreamCreateWithFlags(&side_[q], cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done_[q], cudaEventDisableTiming);
+    }
+    return e;
+  }
+  void destroy() {
+    for (int q = 0; q < 2; ++q) {
+      if (side_[q]) {
+        cudaStreamSynchronize(side_[q]);
+        cudaStreamDestroy(side_[q]);
+      }
+      if (done_[q]) cudaEventDestroy(done_[q]);
+    }
+    if (start_) cudaEventDestroy(start_);
+  }
+  cudaError_t begin(cudaStream_t st) {
+    cudaError_t e = cudaEventRecord(start_, st);
+    for (int q = 0; q < 2 && e == cudaSuccess; ++q) e = cudaStreamWaitEvent(side_[q], start_, 0);
+    return e;
+  }
+  cudaError_t end(cudaStream_t st) {
+    cudaError_t e = cudaSuccess;
+    for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
+      e = cudaEventRecord(done_[q], side_[q]);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, done_[q], 0);
+    }
+    return e;
+  }
+  cudaStream_t side(int q) const { return side_[q]; }
+  StreamPair pair(cudaStream_t st) const { return {st, side_[1]}; }
+
+ private:
+  cudaStream_t side_[2] = {};
+  cudaEvent_t start_ = nullptr, done_[2] = {};
+};
+
 template <typename S> class EngineT : public Engine {
   using R = typename Arith<S>::R;
   friend class BatchT<S>;
@@ -214,9 +258,10 @@ template <typename S> class EngineT : public Engine {
     float amp[343];
     gauss_weights343(amp);
     CUDA_TRY(h2d(amp343_, amp, sizeof amp));
-    // [0] device error flag of the streaming kernel, [1] its work-queue counter
-    CUDA_TRY(cudaMalloc(&err_flag_, 2 * sizeof(int)));
-    CUDA_TRY(cudaMemsetAsync(err_flag_, 0, 2 * sizeof(int), own_stream_));
+    // [0] device error flag of the streaming kernels, [1..4] their two work queues
+    CUDA_TRY(cudaMalloc(&err_flag_, 5 * sizeof(int)));
+    CUDA_TRY(cudaMemsetAsync(err_flag_, 0, 5 * sizeof(int), own_stream_));
+    CUDA_TRY(fork_.create());
     // the device copy of the step counter it_ (read by the per-step kernels)
     CUDA_TRY(cudaMalloc(&step_, 2 * sizeof(int)));  // the step, the end-of-step block counter
     CUDA_TRY(cudaMemsetAsync(step_, 0, 2 * sizeof(int), own_stream_));
@@ -917,12 +962,15 @@ template <typename S> class EngineT : public Engine {
         b0.kend = b1.kend = g_.L.nz_ - HALO - 3;
         b0.chunk = b1.chunk = ch;
         auto pair = [&]() {
-          cudaError_t e = launch_stage_stream<S>(b0, tmap_[0], err_flag_, err_flag_ + 1, st,
-                                                 nullptr, nullptr, rows);
-          if (e == cudaSuccess)
-            e = launch_stage_stream<S>(b1, tmap_[1], err_flag_, err_flag_ + 1, st, nullptr,
-                                       nullptr, rows);
-          return e;
+          for (int q = 0; q < 2; ++q) {
+            cudaError_t e = fork_.begin(st);
+            if (e == cudaSuccess)
+              e = launch_stage_stream<S>(q ? b1 : b0, tmap_[q], err_flag_, err_flag_ + 1,
+                                         fork_.pair(st), nullptr, nullptr, rows);
+            if (e == cudaSuccess) e = fork_.end(st);
+            if (e != cudaSuccess) return e;
+          }
+          return cudaSuccess;
         };
         err = pair();
         if (err == cudaSuccess) err = cudaEventRecord(e0, st);
@@ -973,19 +1021,28 @@ template <typename S> class EngineT : public Engine {
       b.kend = ksurf;
       b.drop_one_load = drop_next_load_ ? 1 : 0;
       drop_next_load_ = false;
-      CUDA_TRY(launch_stage_stream<S>(b, tmap_[in_of[irk]], err_flag_, err_flag_ + 1, st,
+      // The surface, PML and interior launches of a stage write disjoint points
+      // and read none of each other's: the first two run on side streams, so
+      // that they fill the SMs which the others leave idle (timed runs keep
+      // them in turn, to time each).
+      if (!ev) CUDA_TRY(fork_.begin(st));
+      const cudaStream_t side = ev ? st : fork_.side(0);
+      if (!ev) CUDA_TRY(fast_top_ ? launch_surface(&a, 1, side) : launch_surface_exact(a, side));
+      CUDA_TRY(launch_stage_stream<S>(b, tmap_[in_of[irk]], err_flag_, err_flag_ + 1,
+                                      ev ? StreamPair{st, st} : fork_.pair(st),
                                       ev ? ev[1] : nullptr, &launches_,
                                       tile_rows_ ? tile_rows_ : 16));
-      if (ev) CUDA_TRY(cudaEventRecord(ev[2], st));
+      if (ev) {
+        CUDA_TRY(cudaEventRecord(ev[2], st));
+        CUDA_TRY(fast_top_ ? launch_surface(&a, 1, side) : launch_surface_exact(a, side));
+      } else {
+        CUDA_TRY(fork_.end(st));
+      }
       // fields read and written per point by this stage: W in, 12 coefficients,
       // W out, plus m (stages 1, 2), stage 1's input (2) and t (written in 2,
       // read in 3)
       static const int nfield[4] = {30, 39, 57, 39};
       stream_bytes_ += (double)nfield[irk] * sizeof(S) * (double)(g_.nx) * g_.ny * (ksurf - HALO);
-      if (fast_top_)
-        CUDA_TRY(launch_surface(&a, 1, st));
-      else
-        CUDA_TRY(launch_surface_exact(a, st));
     } else {
       if (ev) {
         CUDA_TRY(cudaEventRecord(ev[1], st));
@@ -1097,6 +1154,7 @@ template <typename S> class EngineT : public Engine {
     cudaSetDevice(d_.device);
     if (own_stream_) cudaStreamSynchronize(own_stream_);
     if (last_stream_) cudaStreamSynchronize(last_stream_);
+    fork_.destroy();
     for (void *p : {(void *)A_, (void *)X_, (void *)Y_, (void *)T_, (void *)cjm_, (void *)rdz_,
                     (void *)pml_, (void *)aux_, (void *)pgv_, (void *)amp343_, (void *)sta_xyz_,
                     (void *)sta_wave_, (void *)err_flag_, (void *)step_, (void *)moment_tab_})
@@ -1112,6 +1170,7 @@ template <typename S> class EngineT : public Engine {
   cgfdm_desc d_;
   Dims g_;
   cudaStream_t own_stream_ = nullptr, last_stream_ = nullptr;
+  Fork fork_;
   S *A_ = nullptr, *X_ = nullptr, *Y_ = nullptr, *T_ = nullptr, *cjm_ = nullptr;
   R *rdz_ = nullptr, *pml_ = nullptr, *aux_ = nullptr;
   long long aux_total_ = 0;
@@ -1180,6 +1239,7 @@ template <typename S> class BatchT : public BatchBase {
     for (auto *m : m_)  // the batch's stream goes away with it; its work is done
       if (m->last_stream_ == own_) m->last_stream_ = nullptr;
     drop_graphs();
+    fork_.destroy();
     if (err_) cudaFree(err_);
     if (own_) cudaStreamDestroy(own_);
   }
@@ -1188,8 +1248,9 @@ template <typename S> class BatchT : public BatchBase {
     dev_ = m_[0]->d_.device;
     CUDA_TRY(cudaSetDevice(dev_));
     CUDA_TRY(cudaStreamCreateWithFlags(&own_, cudaStreamNonBlocking));
-    CUDA_TRY(cudaMalloc(&err_, 2 * sizeof(int)));
-    CUDA_TRY(cudaMemsetAsync(err_, 0, 2 * sizeof(int), own_));
+    CUDA_TRY(cudaMalloc(&err_, 5 * sizeof(int)));
+    CUDA_TRY(cudaMemsetAsync(err_, 0, 5 * sizeof(int), own_));
+    CUDA_TRY(fork_.create());
     CUDA_TRY(cudaStreamSynchronize(own_));
     return CGFDM_OK;
   }
@@ -1268,6 +1329,26 @@ template <typename S> class BatchT : public BatchBase {
     std::vector<StageArgs<S>> args;
     std::vector<const void *> maps;
     for (int irk = 0; irk < 4; ++irk) {
+      CUDA_TRY(fork_.begin(st));
+      // the free-surface layers (and members on the exact-order kernel) beside
+      // the streaming launches, as in launch_stage
+      args.clear();
+      for (auto *m : m_) {
+        int fb[3];
+        m->step_fb(irk, fb);
+        if (m->use_stream_) {
+          const StageArgs<S> a = m->batch_stage(irk, fb);
+          if (m->fast_top_)
+            args.push_back(a);
+          else
+            CUDA_TRY(m->launch_surface_exact(a, fork_.side(0)));
+        } else {
+          int rc = m->launch_stage(irk, fb, fork_.side(0), true);
+          if (rc) return rc;
+        }
+      }
+      if (!args.empty())
+        CUDA_TRY(m_[0]->launch_surface(args.data(), (int)args.size(), fork_.side(0)));
       for (int code = 0; code < 8; ++code) {
         args.clear();
         maps.clear();
@@ -1283,24 +1364,9 @@ template <typename S> class BatchT : public BatchBase {
         }
         if (!args.empty())
           CUDA_TRY(launch_stage_stream_batch<S>(args.data(), maps.data(), (int)args.size(), err_,
-                                                err_ + 1, st));
+                                                err_ + 1, fork_.pair(st)));
       }
-      args.clear();
-      for (auto *m : m_) {
-        int fb[3];
-        m->step_fb(irk, fb);
-        if (m->use_stream_) {
-          const StageArgs<S> a = m->batch_stage(irk, fb);
-          if (m->fast_top_)
-            args.push_back(a);
-          else
-            CUDA_TRY(m->launch_surface_exact(a, st));
-        } else {
-          int rc = m->launch_stage(irk, fb, st, true);
-          if (rc) return rc;
-        }
-      }
-      if (!args.empty()) CUDA_TRY(m_[0]->launch_surface(args.data(), (int)args.size(), st));
+      CUDA_TRY(fork_.end(st));
     }
     for (auto *m : m_) {
       int rc = m->step_end(st);
@@ -1345,7 +1411,8 @@ template <typename S> class BatchT : public BatchBase {
   std::vector<EngineT<S> *> m_;
   int dev_ = 0;
   cudaStream_t own_ = nullptr, last_ = nullptr;
-  int *err_ = nullptr;  // [0] error flag, [1] work counter of the batched launches
+  Fork fork_;
+  int *err_ = nullptr;  // [0] error flag, [1..4] work queues of the batched launches
   bool use_graph_ = false;
   cudaGraphExec_t gexec_[8] = {};
   bool gseen_[8] = {};

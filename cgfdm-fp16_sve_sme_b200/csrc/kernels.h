@@ -40,9 +40,16 @@ constexpr int kTilePair = 64;
 // tiles, one CTA per SM), 8 (32 x 8, two CTAs per SM) or kTilePair (16-bit
 // storage: the paired-point kernel on 64 x 8 interior tiles, the 32 x 8 PML
 // variant elsewhere).
+// The launches of a stage that touch no PML slab go to `main`, those that do
+// to `pml` (independent of each other; the same stream runs them in turn).
+struct StreamPair {
+  cudaStream_t main, pml;
+};
+// `work_counter`: four ints, zero before the first launch that uses them (two
+// work queues; every launch leaves its own at zero).
 template <typename S>
 cudaError_t launch_stage_stream(const StageArgs<S> &a, const void *maps, int *err_flag,
-                                int *work_counter, cudaStream_t st,
+                                int *work_counter, StreamPair st,
                                 cudaEvent_t after_main = nullptr, int *nlaunch = nullptr,
                                 int tile_rows = 16);
 // One stage (same irk and MacCormack signs for all) of n scenarios in
@@ -51,7 +58,7 @@ cudaError_t launch_stage_stream(const StageArgs<S> &a, const void *maps, int *er
 // height 16.
 template <typename S>
 cudaError_t launch_stage_stream_batch(const StageArgs<S> *args, const void *const *maps, int n,
-                                      int *err_flag, int *work_counter, cudaStream_t st,
+                                      int *err_flag, int *work_counter, StreamPair st,
                                       int *nlaunch = nullptr);
 template <typename S> bool stage_stream_supported();
 // Encodes the tensor maps the streaming kernel loads its tiles through (the

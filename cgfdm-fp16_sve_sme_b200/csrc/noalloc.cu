@@ -16,9 +16,8 @@
 //   [0, 4)     error flag.  Zero when the module loads; a kernel sets it when a
 //              bounded wait expires; only a call with wait != 0 reads it back
 //              and clears it.
-//   [4, 8)     work-queue counter of the streaming kernel.  It must be zero
-//              when the kernel starts; every call zeroes it (cudaMemsetAsync on
-//              the caller's stream) before every launch.
+//   [4, 20)    the streaming kernels' two work queues.  Zero when the module
+//              loads, and every launch leaves its own at zero.
 //   [256, ...) PML profiles alpha, beta, d for x, y, z (3 x (_nx_+_ny_+_nz_)
 //              floats), rewritten by every call before its launches.  The
 //              values travel in the parameters of small fill kernels on the
@@ -161,7 +160,7 @@ int stage_noalloc(const cgfdm_stage_buffers &b, cudaStream_t st, unsigned char *
     StageArgs<S> lower = a;
     lower.kbeg = HALO;
     lower.kend = ksurf;
-    NA_TRY(launch_stage_stream<S>(lower, maps, err, counter, st));
+    NA_TRY(launch_stage_stream<S>(lower, maps, err, counter, StreamPair{st, st}));
   }
   a.kbeg = ksurf;
   a.kend = L.nz_ - HALO;

@@ -139,6 +139,18 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map
       : "memory");
 }
 
+// End of a launch (thread 0 of each block): the last block to leave sets the
+// work queue back to empty, so that the next launch needs no memset before
+// it.  q[0] is the queue's next item, q[1] the blocks that have left; by then
+// every block has taken its last item.
+__device__ __forceinline__ void queue_leave(int *q) {
+  if (atomicAdd(q + 1, 1) == (int)gridDim.x - 1) {
+    q[0] = 0;
+    q[1] = 0;
+    __threadfence();
+  }
+}
+
 // Elastic combination of one direction from its raw derivatives
 // (wave_deriv.cpp:163-191 without the PML factor): m = metric row,
 // L = d(Vx,Vy,Vz,Txx,Tyy,Tzz,Txy,Txz,Tyz).  Velocity rows include b.
@@ -842,6 +854,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
     fc0 += nout;
     if (ring_m) fm0 += nout;
   }
+  if (tid == 0) queue_leave(src.counter());
 }
 
 template <typename S, int TYv, int FB1, int FB2, int FB3, bool PMLK, int RK>
@@ -1184,6 +1197,7 @@ __global__ void __launch_bounds__(256, 1)
     fc0 += nout;
     if (ring_m) fm0 += nout;
   }
+  if (tid == 0) queue_leave(wk.counter);
 }
 
 // Sets a kernel's dynamic shared-memory limit once per device.  `done` is
@@ -1211,8 +1225,6 @@ cudaError_t launch_variant(const StageArgs<S> &a, const Maps &maps, const Work &
   const int smem = G::SMEM;
   cudaError_t e = ensure_smem_attr(kern, smem, attr_done);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(wk.counter, 0, sizeof(int), st);
-  if (e != cudaSuccess) return e;
   kern<<<std::min(wk.nitems, nsm * G::MINB), G::NTHR, smem, st>>>(maps, a, wk, err);
   return cudaGetLastError();
 }
@@ -1233,13 +1245,14 @@ int sm_count() {
 }
 
 // Item geometry of one stage of one scenario (see Work) and the item counts
-// of its interior and PML launches.
+// of its interior and PML launches; group_tiles: the tiles of all scenarios
+// that share the launches (0: this one alone).
 struct WorkPlan {
   Work wk;
   int n_in, n_pml;
 };
 template <typename S, int TYv>
-WorkPlan plan_work(const StageArgs<S> &a, int nsm, int *counter) {
+WorkPlan plan_work(const StageArgs<S> &a, int nsm, int *counter, int group_tiles = 0) {
   constexpr int TY = TYv;
   constexpr int slots = Geo<S, TYv>::MINB;  // CTAs resident per SM
   const int nx = a.L.nx_ - 2 * HALO, ny = a.L.ny_ - 2 * HALO;
@@ -1268,6 +1281,27 @@ WorkPlan plan_work(const StageArgs<S> &a, int nsm, int *counter) {
   // with chunks of at least 16 planes
   int nic = pl_i > 0 ? (40 * nsm * slots + tiles - 1) / tiles : 0;
   if (pl_i > 0) nic = std::max(1, std::min(nic, pl_i / 16));
+  // Grids whose items would not fill the GPU twice: a launch then lasts as
+  // long as its rounds of items, each its planes plus kLead (four planes of
+  // window and about two of latency), so take the depth with the least of
+  // that, for the bottom planes as well.  64x64x48: 3 planes, one round of 9
+  // instead of 23.
+  const long long all = std::max(tiles, group_tiles), room = (long long)nsm * slots;
+  if (all * (wk.nzc + nic) < 2 * room) {
+    constexpr int kLead = 6;
+    int best = 1 << 30;
+    for (int c = std::max(pl_p, pl_i); c >= 2; --c) {
+      const int nz = (pl_p + c - 1) / c, ni = (pl_i + c - 1) / c;
+      const int rounds = (int)((all * (nz + ni) + room - 1) / room);
+      if (rounds * (c + kLead) < best) {
+        best = rounds * (c + kLead);
+        nic = ni;
+        wk.nzc = nz;
+      }
+    }
+    wk.chunk_p = wk.nzc ? (pl_p + wk.nzc - 1) / wk.nzc : 1;
+    wk.nzc = wk.nzc ? (pl_p + wk.chunk_p - 1) / wk.chunk_p : 0;
+  }
   if (pl_i > 0 && a.chunk > 0) nic = (pl_i + a.chunk - 1) / a.chunk;
   wk.chunk_i = nic ? (pl_i + nic - 1) / nic : 1;
   wk.nic = nic ? (pl_i + wk.chunk_i - 1) / wk.chunk_i : 0;
@@ -1279,21 +1313,22 @@ WorkPlan plan_work(const StageArgs<S> &a, int nsm, int *counter) {
 // PML slab) and the PML launch (the rest), see Work.
 template <typename S, int TYv, int FB1, int FB2, int FB3, int RK>
 cudaError_t launch_one(const StageArgs<S> &a, const Maps &maps, int *err, int *counter,
-                       cudaStream_t st, int *nlaunch) {
+                       StreamPair st, int *nlaunch) {
   const int nsm = sm_count();
   const WorkPlan wp = plan_work<S, TYv>(a, nsm, counter);
   cudaError_t e = cudaSuccess;
   Work wi = wp.wk;
   wi.nitems = wp.n_in;
   if (wi.nitems > 0) {
-    e = launch_variant<S, TYv, FB1, FB2, FB3, false, RK>(a, maps, wi, err, nsm, st);
+    e = launch_variant<S, TYv, FB1, FB2, FB3, false, RK>(a, maps, wi, err, nsm, st.main);
     if (e != cudaSuccess) return e;
     if (nlaunch) ++*nlaunch;
   }
   Work wq = wp.wk;
   wq.nitems = wp.n_pml;
+  wq.counter = counter + 2;
   if (wq.nitems > 0) {
-    e = launch_variant<S, TYv, FB1, FB2, FB3, true, RK>(a, maps, wq, err, nsm, st);
+    e = launch_variant<S, TYv, FB1, FB2, FB3, true, RK>(a, maps, wq, err, nsm, st.pml);
     if (e != cudaSuccess) return e;
     if (nlaunch) ++*nlaunch;
   }
@@ -1307,7 +1342,7 @@ cudaError_t launch_one(const StageArgs<S> &a, const Maps &maps, int *err, int *c
 // included).  16-bit storage only.
 template <typename S, int FB1, int FB2, int FB3, int RK>
 cudaError_t launch_one_pair(const StageArgs<S> &a, const Maps &m8, const Maps &mp, int *err,
-                            int *counter, cudaStream_t st, int *nlaunch) {
+                            int *counter, StreamPair st, int *nlaunch) {
   if constexpr (sizeof(S) != 2) {
     return cudaErrorInvalidValue;
   } else {
@@ -1334,17 +1369,16 @@ cudaError_t launch_one_pair(const StageArgs<S> &a, const Maps &m8, const Maps &m
       auto kern = stage_pair_kernel<S, FB1, FB2, FB3, RK>;
       e = ensure_smem_attr(kern, G::SMEM, attr_done);
       if (e != cudaSuccess) return e;
-      e = cudaMemsetAsync(wi.counter, 0, sizeof(int), st);
-      if (e != cudaSuccess) return e;
-      kern<<<std::min(wi.nitems, nsm), G::NTHR, G::SMEM, st>>>(mp, a, wi, err);
+      kern<<<std::min(wi.nitems, nsm), G::NTHR, G::SMEM, st.main>>>(mp, a, wi, err);
       e = cudaGetLastError();
       if (e != cudaSuccess) return e;
       if (nlaunch) ++*nlaunch;
     }
     Work wq = w;
     wq.nitems = w.nzc * tiles + (tiles - tiles_in) * w.nic;
+    wq.counter = counter + 2;
     if (wq.nitems > 0) {
-      e = launch_variant<S, 8, FB1, FB2, FB3, true, RK>(a, m8, wq, err, nsm, st);
+      e = launch_variant<S, 8, FB1, FB2, FB3, true, RK>(a, m8, wq, err, nsm, st.pml);
       if (e != cudaSuccess) return e;
       if (nlaunch) ++*nlaunch;
     }
@@ -1362,8 +1396,6 @@ cudaError_t launch_batch_variant(const BatchParams<S> &p, int items, int *err, i
   const int smem = G::SMEM;
   cudaError_t e = ensure_smem_attr(kern, smem, attr_done);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(p.counter, 0, sizeof(int), st);
-  if (e != cudaSuccess) return e;
   kern<<<std::min(items, nsm), G::NTHR, smem, st>>>(p, err);
   return cudaGetLastError();
 }
@@ -1372,20 +1404,26 @@ cudaError_t launch_batch_variant(const BatchParams<S> &p, int items, int *err, i
 // scenarios per launch pair (interior items of all of them, then PML items).
 template <typename S, int FB1, int FB2, int FB3, int RK>
 cudaError_t launch_batch(const StageArgs<S> *args, const void *const *maps, int n, int *err,
-                         int *counter, cudaStream_t st, int *nlaunch) {
+                         int *counter, StreamPair st, int *nlaunch) {
   const int nsm = sm_count();
   // the launch parameters (about 19 KB) are assembled in per-thread storage
   static thread_local BatchParams<S> params;
   BatchParams<S> *bp = &params;
   for (int b0 = 0; b0 < n; b0 += kBatchMax) {
     const int nb = std::min(kBatchMax, n - b0);
+    long long tiles = 0;
+    for (int q = 0; q < nb; ++q) {
+      const Layout &L = args[b0 + q].L;
+      tiles += (long long)((L.nx_ - 2 * HALO + TX - 1) / TX) * ((L.ny_ - 2 * HALO + 15) / 16);
+    }
+    tiles = std::min<long long>(tiles, 1 << 30);
     for (int pass = 0; pass < 2; ++pass) {
       std::memset((void *)bp, 0, sizeof(BatchParams<S>));
       int total = 0, m = 0;
       for (int q = 0; q < nb; ++q) {
         const StageArgs<S> &a = args[b0 + q];
         if (a.kend <= a.kbeg) continue;
-        const WorkPlan wp = plan_work<S, 16>(a, nsm, counter);
+        const WorkPlan wp = plan_work<S, 16>(a, nsm, counter, (int)tiles);
         const int cnt = pass == 0 ? wp.n_in : wp.n_pml;
         if (cnt <= 0) continue;
         bp->maps[m] = ((const MapSet *)maps[b0 + q])->ty16;
@@ -1398,10 +1436,10 @@ cudaError_t launch_batch(const StageArgs<S> *args, const void *const *maps, int 
       }
       if (!m) continue;
       bp->n = m;
-      bp->counter = counter;
+      bp->counter = counter + 2 * pass;
       cudaError_t e = pass == 0
-                          ? launch_batch_variant<S, FB1, FB2, FB3, false, RK>(*bp, total, err, nsm, st)
-                          : launch_batch_variant<S, FB1, FB2, FB3, true, RK>(*bp, total, err, nsm, st);
+                          ? launch_batch_variant<S, FB1, FB2, FB3, false, RK>(*bp, total, err, nsm, st.main)
+                          : launch_batch_variant<S, FB1, FB2, FB3, true, RK>(*bp, total, err, nsm, st.pml);
       if (e != cudaSuccess) return e;
       if (nlaunch) ++*nlaunch;
     }
@@ -1465,10 +1503,10 @@ int encode_stream_maps<double>(const double *, const double *, const double *, c
                                const double *, const Layout &, void *);
 template <>
 cudaError_t launch_stage_stream_batch<double>(const StageArgs<double> *, const void *const *, int,
-                                              int *, int *, cudaStream_t, int *);
+                                              int *, int *, StreamPair, int *);
 template <>
 cudaError_t launch_stage_stream<double>(const StageArgs<double> &, const void *, int *, int *,
-                                        cudaStream_t, cudaEvent_t, int *, int);
+                                        StreamPair, cudaEvent_t, int *, int);
 
 template <typename S>
 int encode_stream_maps(const S *wave, const S *cjm, const S *wm, const S *t, const S *x,
@@ -1506,7 +1544,7 @@ inline int rk_class(int irk, int lean) {
 
 template <typename S, int TYv, int RK>
 cudaError_t launch_fb_rk(const StageArgs<S> &a, const Maps &m, int *err, int *counter,
-                         cudaStream_t st, int *nlaunch) {
+                         StreamPair st, int *nlaunch) {
   const int code = (a.fb1 > 0) * 4 + (a.fb2 > 0) * 2 + (a.fb3 > 0);
   switch (code) {
     case 0: return launch_one<S, TYv, -1, -1, -1, RK>(a, m, err, counter, st, nlaunch);
@@ -1521,7 +1559,7 @@ cudaError_t launch_fb_rk(const StageArgs<S> &a, const Maps &m, int *err, int *co
 }
 template <typename S, int RK>
 cudaError_t launch_fb_rk_pair(const StageArgs<S> &a, const MapSet &ms, int *err, int *counter,
-                              cudaStream_t st, int *nlaunch) {
+                              StreamPair st, int *nlaunch) {
   const Maps &m8 = ms.ty8, &mp = ms.pair;
   switch ((a.fb1 > 0) * 4 + (a.fb2 > 0) * 2 + (a.fb3 > 0)) {
     case 0: return launch_one_pair<S, -1, -1, -1, RK>(a, m8, mp, err, counter, st, nlaunch);
@@ -1540,7 +1578,7 @@ cudaError_t launch_fb_rk_pair(const StageArgs<S> &a, const MapSet &ms, int *err,
 // STREAM_INSTANTIATE).
 template <typename S, int RK>
 cudaError_t launch_single_rk(const StageArgs<S> &a, const void *maps, int *err, int *counter,
-                             cudaStream_t st, int *nlaunch, int tile_rows) {
+                             StreamPair st, int *nlaunch, int tile_rows) {
   const MapSet &ms = *(const MapSet *)maps;
   if (tile_rows == 8) return launch_fb_rk<S, 8, RK>(a, ms.ty8, err, counter, st, nlaunch);
   if constexpr (sizeof(S) == 2) {
@@ -1550,7 +1588,7 @@ cudaError_t launch_single_rk(const StageArgs<S> &a, const void *maps, int *err, 
 }
 template <typename S, int RK>
 cudaError_t launch_batch_rk(const StageArgs<S> *args, const void *const *maps, int n, int *err,
-                            int *counter, cudaStream_t st, int *nlaunch) {
+                            int *counter, StreamPair st, int *nlaunch) {
   const StageArgs<S> &a = args[0];
   switch ((a.fb1 > 0) * 4 + (a.fb2 > 0) * 2 + (a.fb3 > 0)) {
     case 0: return launch_batch<S, -1, -1, -1, RK>(args, maps, n, err, counter, st, nlaunch);
@@ -1566,9 +1604,9 @@ cudaError_t launch_batch_rk(const StageArgs<S> *args, const void *const *maps, i
 
 #define STREAM_CLASS(EXT, S, RK)                                                                  \
   EXT template cudaError_t launch_single_rk<S, RK>(const StageArgs<S> &, const void *, int *,     \
-                                                   int *, cudaStream_t, int *, int);              \
+                                                   int *, StreamPair, int *, int);                \
   EXT template cudaError_t launch_batch_rk<S, RK>(const StageArgs<S> *, const void *const *, int, \
-                                                  int *, int *, cudaStream_t, int *);
+                                                  int *, int *, StreamPair, int *);
 // The classes of a storage type over three translation units: part 0 the
 // single-stage forms and the dispatch, parts 1 and 2 whole steps.
 #if STREAM_PART == 0
@@ -1584,7 +1622,7 @@ cudaError_t launch_batch_rk(const StageArgs<S> *args, const void *const *maps, i
 
 template <typename S>
 cudaError_t launch_stage_stream(const StageArgs<S> &a, const void *maps_in, int *err, int *counter,
-                                cudaStream_t st, cudaEvent_t after_main, int *nlaunch,
+                                StreamPair st, cudaEvent_t after_main, int *nlaunch,
                                 int tile_rows) {
   if (a.kend <= a.kbeg) return cudaSuccess;
   // tile height 16 runs the batched kernel as a batch of one, so that a
@@ -1603,12 +1641,12 @@ cudaError_t launch_stage_stream(const StageArgs<S> &a, const void *maps_in, int 
     }
   }
   if (e != cudaSuccess) return e;
-  if (after_main) e = cudaEventRecord(after_main, st);
+  if (after_main) e = cudaEventRecord(after_main, st.main);
   return e;
 }
 template <typename S>
 cudaError_t launch_stage_stream_batch(const StageArgs<S> *args, const void *const *maps, int n,
-                                      int *err, int *counter, cudaStream_t st, int *nlaunch) {
+                                      int *err, int *counter, StreamPair st, int *nlaunch) {
   if (n <= 0) return cudaSuccess;
   for (int q = 1; q < n; ++q)
     if (args[q].fb1 != args[0].fb1 || args[q].fb2 != args[0].fb2 || args[q].fb3 != args[0].fb3 ||

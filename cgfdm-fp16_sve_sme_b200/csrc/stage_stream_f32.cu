@@ -19,24 +19,24 @@ int encode_stream_maps<double>(const double *, const double *, const double *, c
 
 template <>
 cudaError_t launch_stage_stream_batch<double>(const StageArgs<double> *, const void *const *, int,
-                                              int *, int *, cudaStream_t, int *) {
+                                              int *, int *, StreamPair, int *) {
   return cudaErrorNotSupported;
 }
 
 template <>
 cudaError_t launch_stage_stream<double>(const StageArgs<double> &, const void *, int *, int *,
-                                        cudaStream_t, cudaEvent_t, int *, int) {
+                                        StreamPair, cudaEvent_t, int *, int) {
   return cudaErrorNotSupported;
 }
 
 template cudaError_t launch_stage_stream_batch<float>(const StageArgs<float> *,
                                                       const void *const *, int, int *, int *,
-                                                      cudaStream_t, int *);
+                                                      StreamPair, int *);
 template bool stage_stream_supported<float>();
 template int encode_stream_maps<float>(const float *, const float *, const float *, const float *,
                                        const float *, const Layout &, void *);
 template cudaError_t launch_stage_stream<float>(const StageArgs<float> &, const void *, int *,
-                                                int *, cudaStream_t, cudaEvent_t, int *, int);
+                                                int *, StreamPair, cudaEvent_t, int *, int);
 
 #endif
 

@@ -341,9 +341,9 @@ int cgfdm_server_destroy(cgfdm_server *s);
  *
  * Limits and rules: precision FP32, FP16 or BF16; the PML profile table must
  * fit the scratch (nx + ny + nz + 18 <= 5440, else CGFDM_ERR_ARG).  All calls
- * on one device share the scratch and see what the last call left there:
- * each call zeroes the work-queue counter itself, so calls whose work
- * overlaps on the GPU race.  The error flag starts at zero, is set by an
+ * on one device share the scratch and see what the last call left there
+ * (every launch leaves its work queue empty), so calls whose work overlaps
+ * on the GPU race.  The error flag starts at zero, is set by an
  * expired bounded wait, and is read and cleared only when `wait` is
  * non-zero: then the call synchronizes `stream` and returns CGFDM_ERR_TIMEOUT
  * if it was set.  With wait = 0 the call only enqueues work on `stream`
