@@ -105,6 +105,19 @@ __global__ void slice_pack_kernel(const S *f, Layout L, int axis, int at, double
   out[t] = (float)((double)(float)ldv(f + L.at(i, j, k)) * c);
 }
 
+// Pad and halo cells included: they are zero or the caller's values.
+template <typename S>
+__global__ void lateral_check_kernel(const S *cjm, long long fs, int *flag) {
+  using R = typename Arith<S>::R;
+  const int f[4] = {1, 2, 3, 5};
+  bool any = false;
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < fs;
+       q += (long long)gridDim.x * blockDim.x)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) any = any || !((R)ldv(cjm + f[v] * fs + q) == (R)0.0f);
+  if (any) *flag = 1;
+}
+
 template <typename S>
 __global__ void repack_in_kernel(const float *src, S *dst, Layout L, int nfield) {
   const long long num = (long long)L.nx_ * L.ny_ * L.nz_;
@@ -171,6 +184,12 @@ cudaError_t launch_slice_pack(const S *field, Layout L, int axis, int at, double
 }
 
 template <typename S>
+cudaError_t launch_lateral_check(const S *cjm, Layout L, int *flag, cudaStream_t st) {
+  lateral_check_kernel<S><<<1184, 256, 0, st>>>(cjm, L.fs, flag);
+  return cudaGetLastError();
+}
+
+template <typename S>
 cudaError_t launch_repack_in(const float *src, S *dst, Layout L, int nfield, cudaStream_t st) {
   repack_in_kernel<S><<<2368, 256, 0, st>>>(src, dst, L, nfield);
   return cudaGetLastError();
@@ -193,6 +212,7 @@ cudaError_t launch_repack_out(const S *src, float *dst, Layout L, int nfield, cu
                                              cudaStream_t);                                        \
   template cudaError_t launch_slice_pack<S>(const S *, Layout, int, int, double, float *,         \
                                             cudaStream_t);                                         \
+  template cudaError_t launch_lateral_check<S>(const S *, Layout, int *, cudaStream_t);            \
   template cudaError_t launch_repack_in<S>(const float *, S *, Layout, int, cudaStream_t);        \
   template cudaError_t launch_repack_out<S>(const S *, float *, Layout, int, cudaStream_t);
 

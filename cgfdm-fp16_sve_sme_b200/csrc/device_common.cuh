@@ -120,6 +120,12 @@ template <typename S> struct StageArgs {
   // (the auxiliaries alike).  165 instead of 192 fields move per point and
   // step, and t is rounded once instead of three times.
   int lean;
+  // 1: xi_y, xi_z, eta_x and eta_z are zero in every cell (a grid stretched in
+  // z only, which every grid built from a run directory is) and the stage is
+  // one of a whole step: the streaming kernels neither load these four fields
+  // nor form what they would multiply.  Finite fields give the same values;
+  // an infinity or NaN spreads through the other metrics' terms only.
+  int vert;
   // planes per upper z chunk of the streaming kernel's work items (0: about
   // 40 items per CTA slot, chunks of at least 16 planes)
   int chunk;

@@ -258,9 +258,10 @@ template <typename S> class EngineT : public Engine {
     float amp[343];
     gauss_weights343(amp);
     CUDA_TRY(h2d(amp343_, amp, sizeof amp));
-    // [0] device error flag of the streaming kernels, [1..4] their two work queues
-    CUDA_TRY(cudaMalloc(&err_flag_, 5 * sizeof(int)));
-    CUDA_TRY(cudaMemsetAsync(err_flag_, 0, 5 * sizeof(int), own_stream_));
+    // [0] device error flag of the streaming kernels, [1..4] their two work
+    // queues, [5] set_model's check
+    CUDA_TRY(cudaMalloc(&err_flag_, 6 * sizeof(int)));
+    CUDA_TRY(cudaMemsetAsync(err_flag_, 0, 6 * sizeof(int), own_stream_));
     CUDA_TRY(fork_.create());
     // the device copy of the step counter it_ (read by the per-step kernels)
     CUDA_TRY(cudaMalloc(&step_, 2 * sizeof(int)));  // the step, the end-of-step block counter
@@ -295,6 +296,15 @@ template <typename S> class EngineT : public Engine {
     int rc = synchronize();  // no stage of this handle may be reading the coefficients
     if (rc) return rc;
     CUDA_TRY(upload_through_accumulator(cjm, cjm_, 13));
+    // a grid stretched in z only takes the streaming kernels' shorter form
+    int lateral = 0;
+    CUDA_TRY(cudaMemsetAsync(err_flag_ + 5, 0, sizeof(int), own_stream_));
+    CUDA_TRY(launch_lateral_check<S>(cjm_, g_.L, err_flag_ + 5, own_stream_));
+    CUDA_TRY(cudaMemcpyAsync(&lateral, err_flag_ + 5, sizeof(int), cudaMemcpyDeviceToHost,
+                             own_stream_));
+    CUDA_TRY(cudaStreamSynchronize(own_stream_));
+    vert_ = lateral == 0;
+    drop_graphs();
     std::vector<R> r(rdz, rdz + 18 * g_.nsurf);
     CUDA_TRY(h2d(rdz_, r.data(), sizeof(R) * r.size()));
     host_cjm_J_.assign(cjm + 9 * g_.num, cjm + 10 * g_.num);
@@ -892,6 +902,7 @@ template <typename S> class EngineT : public Engine {
     a.fb1 = fb[0]; a.fb2 = fb[1]; a.fb3 = fb[2];
     a.irk = irk;
     a.lean = whole_step && use_stream_ ? 1 : 0;
+    a.vert = a.lean && vert_ ? 1 : 0;
     a.chunk = chunk_;
     a.nslab = g_.npml > 0 ? 5 : 0;
     size_t off = 0;
@@ -1038,11 +1049,11 @@ template <typename S> class EngineT : public Engine {
       } else {
         CUDA_TRY(fork_.end(st));
       }
-      // fields read and written per point by this stage: W in, 12 coefficients,
-      // W out, plus m (stages 1, 2), stage 1's input (2) and t (written in 2,
-      // read in 3)
+      // fields read and written per point by this stage: W in, 12 coefficients
+      // (8 on a vertically stretched grid), W out, plus m (stages 1, 2), stage
+      // 1's input (2) and t (written in 2, read in 3)
       static const int nfield[4] = {30, 39, 57, 39};
-      stream_bytes_ += (double)nfield[irk] * sizeof(S) * (double)(g_.nx) * g_.ny * (ksurf - HALO);
+      stream_bytes_ += (double)(nfield[irk] - (a.vert ? 4 : 0)) * sizeof(S) * (double)(g_.nx) * g_.ny * (ksurf - HALO);
     } else {
       if (ev) {
         CUDA_TRY(cudaEventRecord(ev[1], st));
@@ -1143,6 +1154,7 @@ template <typename S> class EngineT : public Engine {
   }
 
   void drop_graphs() {
+    ++rev_;
     for (int p = 0; p < 8; ++p) {
       if (gexec_[p]) cudaGraphExecDestroy(gexec_[p]);
       gexec_[p] = nullptr;
@@ -1195,6 +1207,8 @@ template <typename S> class EngineT : public Engine {
   int launches_ = 0;          // kernels launched by the last run()
   int tile_rows_ = 0;         // streaming-kernel tile height; 0 = autotune at the first run()
   int chunk_ = 0;             // planes per streaming work item in z; 0 = automatic
+  bool vert_ = false;         // see StageArgs::vert; false until a model is set
+  unsigned rev_ = 0;          // counts what makes captured steps stale
   bool fast_top_ = true;      // free-surface layers on the tiled kernel (see Tuned)
   bool chunk_fixed_ = false;  // set by set_chunk: the autotuner keeps chunk_
   bool drop_next_load_ = false;  // fault injection for failure-detection tests
@@ -1285,6 +1299,14 @@ template <typename S> class BatchT : public BatchBase {
         }
       tuned_ = true;
     }
+    // a member whose model, sources, stations or form changed makes the
+    // captured steps stale
+    std::vector<unsigned> revs;
+    for (auto *m : m_) revs.push_back(m->rev_);
+    if (revs != revs_) {
+      drop_graphs();
+      revs_ = revs;
+    }
     for (int s = 0; s < nsteps; ++s) {
       const int p = count_ % 8;
       if (use_graph_) {
@@ -1349,13 +1371,15 @@ template <typename S> class BatchT : public BatchBase {
       }
       if (!args.empty())
         CUDA_TRY(m_[0]->launch_surface(args.data(), (int)args.size(), fork_.side(0)));
-      for (int code = 0; code < 8; ++code) {
+      for (int code = 0; code < 16; ++code) {
         args.clear();
         maps.clear();
         for (auto *m : m_) {
           int fb[3];
           m->step_fb(irk, fb);
-          if (!m->use_stream_ || (fb[0] > 0) * 4 + (fb[1] > 0) * 2 + (fb[2] > 0) != code) continue;
+          if (!m->use_stream_ ||
+              m->vert_ * 8 + (fb[0] > 0) * 4 + (fb[1] > 0) * 2 + (fb[2] > 0) != code)
+            continue;
           StageArgs<S> a = m->stage_args(irk, fb, true);
           a.kbeg = HALO;
           a.kend = m->g_.L.nz_ - HALO - 3;
@@ -1417,6 +1441,7 @@ template <typename S> class BatchT : public BatchBase {
   cudaGraphExec_t gexec_[8] = {};
   bool gseen_[8] = {};
   long long count_ = 0;  // steps run by this batch
+  std::vector<unsigned> revs_;  // members' rev_ when the graphs were captured
   bool tuned_ = false;   // members' work-item depths chosen (first run)
 };
 

@@ -105,6 +105,11 @@ template <typename S>
 cudaError_t launch_slice_pack(const S *field, Layout L, int axis, int at, double c, float *out,
                               cudaStream_t st);
 
+// Sets *flag to 1 if one of the fields xi_y, xi_z, eta_x, eta_z of `cjm` has a
+// nonzero value (see StageArgs::vert).
+template <typename S>
+cudaError_t launch_lateral_check(const S *cjm, Layout L, int *flag, cudaStream_t st);
+
 // Reference layout (float, nfield x num) <-> HBM layout (S, nfield x fs).
 template <typename S>
 cudaError_t launch_repack_in(const float *src, S *dst, Layout L, int nfield, cudaStream_t st);

@@ -11,12 +11,12 @@
 // it: a 5-plane register window per thread holds the z stencil, and shared
 // memory holds three rings fed by 4-D TMA tile loads (cp.async.bulk.tensor,
 // no multicast), each slot guarded by an mbarrier:
-//   W ring (3): the 9 wavefield components of one input plane with the x/y
+//   W ring (4): the 9 wavefield components of one input plane with the x/y
 //               halo of the one-sided stencils (x origin 16-byte aligned);
 //   C ring (2): the 9 metrics and (mu, lambda, buoyancy) of one output plane;
 //   M ring (2): the RK step state m and accumulator t (or what t is formed
 //               from) of one output plane (stages that read them);
-// (4/3/3 slots in the 16-bit PML variant, see Geo).
+// (the depths are those of FP32 in 32 x 16 tiles, see Rings).
 // With 16-bit storage the interior variant converts each W plane to FP32 once
 // in shared memory (two plane buffers), so its stencils read FP32 like the
 // FP32 kernel instead of converting every tap.
@@ -58,35 +58,62 @@ namespace {
 constexpr int TX = 32;
 constexpr long long kWaitCycles = 1LL << 31;
 
-// Tile and shared-memory geometry for storage type S and tile height TYv
-// (16: one 512-thread CTA per SM; 8: 256-thread CTAs, two per SM when their
-// shared memory fits, so one CTA's per-plane barrier overlaps the other's work).
-template <typename S, int TYv, bool PMLK = false> struct Geo {
+// Stage classes RK of the kernels: 0, 1 (stages 1 and 2) and 3 update the
+// accumulator as the reference does; 4, 5 and 6 are stages 0, 1 and 2 of a
+// whole step (StageArgs::lean), whose stage 3 is class 3 too.  Compile-time
+// classes: with the form chosen at run time the PML variant of stages 1-2
+// spilled 28-60 bytes a thread at its 128 registers.
+enum { kTsAcc = 0, kTsNone = 1, kTsOld = 2 };  // what t comes from, if it is written
+template <int RK> constexpr int stage_of() { return RK == 4 ? 0 : RK >= 5 ? 1 : RK; }
+template <int RK> constexpr int tsel_of() {
+  return RK == 4 || RK == 5 ? kTsNone : RK == 6 ? kTsOld : kTsAcc;
+}
+
+// Tile geometry for storage type S and tile height TYv (16: one 512-thread
+// CTA per SM; 8: 256-thread CTAs, two per SM, so one CTA's per-plane barrier
+// overlaps the other's work).
+template <typename S, int TYv> struct Geo {
   static constexpr int TY = TYv, NTHR = TX * TYv;
   static constexpr int BY = TYv + 4;  // y box: 1 or 3 rows before the tile, 3 or 1 after
   static constexpr int MINB = TYv == 8 ? 2 : 1;
   static constexpr int ES = (int)sizeof(S);
   static constexpr int HB = 16 / ES;                             // elements per 16 bytes
   static constexpr int BX = ((HB + TX + 3) + HB - 1) / HB * HB;  // x box, aligned origin
-  static constexpr int W_BYTES = ((9 * BY * BX * ES) + 127) / 128 * 128;
-  static constexpr int C_BYTES = 12 * NTHR * ES;                 // 9 metrics + mu, lambda, b
-  static constexpr int M_BYTES = 18 * NTHR * ES;                 // m (9) and t (9)
+};
+// Shared-memory rings of one kernel.  VT: see StageArgs::vert (8 coefficient
+// fields instead of 12).  The m/t ring holds what the stage class reads, and
+// what that leaves of the shared memory goes to the W ring (at most kMaxW
+// planes), whose loads run ahead of the sweep.
+constexpr int kMaxW = 5;
+template <typename S, int TYv, bool PMLK, int RK, bool VT> struct Rings : Geo<S, TYv> {
+  using B = Geo<S, TYv>;
+  static constexpr int NTHR = B::NTHR, ES = B::ES;
+  static constexpr int W_BYTES = ((9 * B::BY * B::BX * ES) + 127) / 128 * 128;
+  static constexpr int CF = VT ? 8 : 12;  // metrics, mu, lambda, b
+  static constexpr int MF = (stage_of<RK>() == 1 ? 9 : 0) +
+                            (stage_of<RK>() >= 1 && tsel_of<RK>() != kTsNone ? 9 : 0);
+  static constexpr int C_BYTES = CF * NTHR * ES;
+  static constexpr int M_BYTES = MF * NTHR * ES;  // m (9) and t (9), those that are read
+  static constexpr int T_AT = stage_of<RK>() == 1 ? 9 : 0;  // first field of t in a slot
   // 16-bit storage, interior variant: each W plane is converted to FP32 once,
   // into one of two plane buffers (by plane parity) that the x and y stencils
   // read.  The PML variant (latency-bound) reads the 16-bit planes directly
   // and keeps deeper rings instead.
   static constexpr bool CONV = ES != 4 && !PMLK;
-  static constexpr int NW = ES == 4 || CONV ? 3 : 4;
   static constexpr int NC = ES == 4 || CONV ? 2 : 3;
   static constexpr int NM = NC;
-  static constexpr int F_BYTES = CONV ? ((9 * BY * BX * 4) + 127) / 128 * 128 : 0;
+  static constexpr int F_BYTES = CONV ? ((9 * B::BY * B::BX * 4) + 127) / 128 * 128 : 0;
+  static constexpr int ROOM = (B::MINB == 1 ? 232448 : 233472 / B::MINB - 1024) - 512 -
+                              NC * C_BYTES - NM * M_BYTES - 2 * F_BYTES;
+  static constexpr int NW = ROOM / W_BYTES < kMaxW ? ROOM / W_BYTES : kMaxW;
   static constexpr int OFF_C = NW * W_BYTES;
   static constexpr int OFF_M = OFF_C + NC * C_BYTES;
   static constexpr int OFF_F = OFF_M + NM * M_BYTES;
   static constexpr int OFF_BAR = OFF_F + 2 * F_BYTES;
   static constexpr int SMEM = OFF_BAR + 8 * (NW + NC + NM) + 128;
+  static_assert(NW >= 3, "W ring");
   static_assert(SMEM <= 232448, "shared memory budget");
-  static_assert(MINB == 1 || MINB * (SMEM + 1024) <= 233472, "two CTAs per SM");
+  static_assert(B::MINB == 1 || B::MINB * (SMEM + 1024) <= 233472, "two CTAs per SM");
 };
 
 // Four 16-bit values at p (8-byte aligned) as four floats.
@@ -153,21 +180,40 @@ __device__ __forceinline__ void queue_leave(int *q) {
 
 // Elastic combination of one direction from its raw derivatives
 // (wave_deriv.cpp:163-191 without the PML factor): m = metric row,
-// L = d(Vx,Vy,Vz,Txx,Tyy,Tzz,Txy,Txz,Tyz).  Velocity rows include b.
+// L = d(Vx,Vy,Vz,Txx,Tyy,Tzz,Txy,Txz,Tyz).  Velocity rows include b.  Here
+// and in the auxiliary update every contraction is written out, so that all
+// kernels that compute a point give the same bits.
 __device__ __forceinline__ void elastic9(const float m[3], const float L[9], float mu, float lam,
                                          float b, float E[9]) {
-  E[0] = (m[0] * L[3] + m[1] * L[6] + m[2] * L[7]) * b;
-  E[1] = (m[0] * L[6] + m[1] * L[4] + m[2] * L[8]) * b;
-  E[2] = (m[0] * L[7] + m[1] * L[8] + m[2] * L[5]) * b;
-  const float mvx = m[0] * L[0], mvy = m[1] * L[1], mvz = m[2] * L[2];
-  const float div = (mvx + mvy + mvz) * lam;
+  E[0] = fmaf(m[2], L[7], fmaf(m[1], L[6], m[0] * L[3])) * b;
+  E[1] = fmaf(m[2], L[8], fmaf(m[1], L[4], m[0] * L[6])) * b;
+  E[2] = fmaf(m[2], L[5], fmaf(m[1], L[8], m[0] * L[7])) * b;
+  const float mvx = __fmul_rn(m[0], L[0]), mvy = __fmul_rn(m[1], L[1]), mvz = __fmul_rn(m[2], L[2]);
+  const float div = __fmul_rn(__fadd_rn(__fadd_rn(mvx, mvy), mvz), lam);
   const float tmu = 2.0f * mu;
-  E[3] = div + tmu * mvx;
-  E[4] = div + tmu * mvy;
-  E[5] = div + tmu * mvz;
-  E[6] = (m[1] * L[0] + m[0] * L[1]) * mu;
-  E[7] = (m[2] * L[0] + m[0] * L[2]) * mu;
-  E[8] = (m[2] * L[1] + m[1] * L[2]) * mu;
+  E[3] = fmaf(tmu, mvx, div);
+  E[4] = fmaf(tmu, mvy, div);
+  E[5] = fmaf(tmu, mvz, div);
+  E[6] = fmaf(m[1], L[0], m[0] * L[1]) * mu;
+  E[7] = fmaf(m[2], L[0], m[0] * L[2]) * mu;
+  E[8] = fmaf(m[2], L[1], m[1] * L[2]) * mu;
+}
+// The same with one metric of the row alone, its x (AX = 0) or y (AX = 1)
+// component g; the terms of the others are zero (StageArgs::vert).
+template <int AX>
+__device__ __forceinline__ void elastic9_vert(float g, const float L[9], float mu, float lam,
+                                              float b, float E[9]) {
+  E[0] = g * L[AX ? 6 : 3] * b;
+  E[1] = g * L[AX ? 4 : 6] * b;
+  E[2] = g * L[AX ? 8 : 7] * b;
+  const float gv = __fmul_rn(g, L[AX]);
+  const float div = __fmul_rn(gv, lam), two = fmaf(2.0f * mu, gv, div);
+  E[3] = AX ? div : two;
+  E[4] = AX ? two : div;
+  E[5] = div;
+  E[6] = g * L[AX ? 0 : 1] * mu;
+  E[7] = AX ? 0.0f : g * L[2] * mu;
+  E[8] = AX ? g * L[2] * mu : 0.0f;
 }
 
 // The interior variant's form of the three directions' elastic combinations
@@ -193,6 +239,27 @@ struct ElasticSum {
     s6 = fmaf(a0, L[1], FIRST ? a1 * L[0] : fmaf(a1, L[0], s6));
     s7 = fmaf(a0, L[2], FIRST ? a2 * L[0] : fmaf(a2, L[0], s7));
     s8 = fmaf(a1, L[2], FIRST ? a2 * L[1] : fmaf(a2, L[1], s8));
+  }
+  // x direction first, then y, with xi_x (eta_y) the only metric of the row
+  __device__ __forceinline__ void add_vert_x(float m, float g, const float L[9]) {
+    const float a = g * m;
+    v0 = a * L[3];
+    v1 = a * L[6];
+    v2 = a * L[7];
+    nx = a * L[0];
+    ny = nz = 0.0f;
+    s6 = a * L[1];
+    s7 = a * L[2];
+    s8 = 0.0f;
+  }
+  __device__ __forceinline__ void add_vert_y(float m, float g, const float L[9]) {
+    const float a = g * m;
+    v0 = fmaf(a, L[6], v0);
+    v1 = fmaf(a, L[4], v1);
+    v2 = fmaf(a, L[8], v2);
+    ny = a * L[1];
+    s6 = fmaf(a, L[0], s6);
+    s8 = a * L[2];
   }
   __device__ __forceinline__ void finish(float mu, float lam, float b, float h[9]) const {
     h[0] = v0 * b;
@@ -227,17 +294,6 @@ __device__ __forceinline__ float2 stencil2(float2 t0, float2 t1, float2 t2, floa
 }
 __device__ __forceinline__ float stencil1(float t0, float t1, float t2, float t3, float t4) {
   return fmaf(kA3, t4, fmaf(kA2, t3, fmaf(kA1, t2, fmaf(kA0, t1, kAm1 * t0))));
-}
-
-// Stage classes RK of the kernels: 0, 1 (stages 1 and 2) and 3 update the
-// accumulator as the reference does; 4, 5 and 6 are stages 0, 1 and 2 of a
-// whole step (StageArgs::lean), whose stage 3 is class 3 too.  Compile-time
-// classes: with the form chosen at run time the PML variant of stages 1-2
-// spilled 28-60 bytes a thread at its 128 registers.
-enum { kTsAcc = 0, kTsNone = 1, kTsOld = 2 };  // what t comes from, if it is written
-template <int RK> constexpr int stage_of() { return RK == 4 ? 0 : RK >= 5 ? 1 : RK; }
-template <int RK> constexpr int tsel_of() {
-  return RK == 4 || RK == 5 ? kTsNone : RK == 6 ? kTsOld : kTsAcc;
 }
 
 // t from the step state m, the inputs w1 and w2 of stages 1 and 2 and stage
@@ -325,18 +381,19 @@ __device__ __forceinline__ void pml_apply(const SlabDev<float> &sl, unsigned pos
     for (int v = g; v < g + 3; ++v) {
       const unsigned q = v * np + pos;
       const float a = in.a[v];
-      const float ha = (dl * E[v] - ad * a) * DT;
-      h[v] -= bt * a * DT;
+      const float ha = __fmul_rn(fmaf(dl, E[v], -__fmul_rn(ad, a)), DT);
+      h[v] = fmaf(-__fmul_rn(bt, a), DT, h[v]);
       if (ST == 0) {
-        if (tsel == kTsAcc) at[q] = a + kB1 * ha;
-        aout[q] = a + kA2rk * ha;
+        if (tsel == kTsAcc) at[q] = fmaf(kB1, ha, a);
+        aout[q] = fmaf(kA2rk, ha, a);
       } else if (ST == 1) {
         const float m = in.b[v];
-        if (tsel == kTsAcc) at[q] = in.t[v] + cB * ha;
-        if (tsel == kTsOld) at[q] = m + (kT1 * (in.t[v] - m) + (kT2 * (a - m) + cB * ha));
-        aout[q] = m + cA * ha;
+        if (tsel == kTsAcc) at[q] = fmaf(cB, ha, in.t[v]);
+        if (tsel == kTsOld)
+          at[q] = __fadd_rn(m, fmaf(kT1, in.t[v] - m, fmaf(kT2, a - m, __fmul_rn(cB, ha))));
+        aout[q] = fmaf(cA, ha, m);
       } else {
-        aout[q] = in.b[v] + kB4 * ha;
+        aout[q] = fmaf(kB4, ha, in.b[v]);
       }
     }
   }
@@ -352,6 +409,7 @@ struct Maps {
   CUtensorMap w;   // stage input wavefield, box BX x BY x 1 x 9
   CUtensorMap c9;  // coefficients, box 32 x TY x 1 x 9 (metrics)
   CUtensorMap c3;  // coefficients, box 32 x TY x 1 x 3 (mu, lambda, b at field 10)
+  CUtensorMap c1;  // coefficients, box 32 x TY x 1 x 1 (StageArgs::vert)
   CUtensorMap m;   // step-start wavefield, box 32 x TY x 1 x 9
   CUtensorMap t;   // RK accumulator, box 32 x TY x 1 x 9
   CUtensorMap x;   // stage output before the stage, box 32 x TY x 1 x 9
@@ -468,9 +526,25 @@ template <typename S> struct BatchSrc {
   __device__ const Work &work(int e) const { return p.work[e]; }
 };
 
-template <typename S, int TYv, int FB1, int FB2, int FB3, bool PMLK, int RK, typename Src>
+// One plane's coefficients into smem (dst, bytes per field fb): all 12, or of
+// a vertically stretched grid xi_x, eta_y, the zeta row and mu, lambda, b.
+template <bool VT>
+__device__ __forceinline__ void load_coefs(const Maps &maps, uint32_t dst, int fb, int x, int y,
+                                           int z, uint32_t bar) {
+  if (VT) {
+    tma_load_4d(dst, &maps.c1, x, y, z, 0, bar);
+    tma_load_4d(dst + fb, &maps.c1, x, y, z, 4, bar);
+    tma_load_4d(dst + 2 * fb, &maps.c3, x, y, z, 6, bar);
+    tma_load_4d(dst + 5 * fb, &maps.c3, x, y, z, 10, bar);
+  } else {
+    tma_load_4d(dst, &maps.c9, x, y, z, 0, bar);
+    tma_load_4d(dst + 9 * fb, &maps.c3, x, y, z, 10, bar);
+  }
+}
+
+template <typename S, int TYv, int FB1, int FB2, int FB3, bool PMLK, int RK, bool VT, typename Src>
 __device__ __forceinline__ void stream_body(const Src &src, int *err) {
-  using G = Geo<S, TYv, PMLK>;
+  using G = Rings<S, TYv, PMLK, RK, VT>;
   constexpr int TY = G::TY, NTHR = G::NTHR, BY = G::BY;
   constexpr int NW = G::NW, NC = G::NC, NM = G::NM, BX = G::BX;
   constexpr int DIR = -FB3;  // sweep direction in z
@@ -547,8 +621,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
       const uint32_t bar = smem_u32(&bc[s]);
       unsigned char *dst = smem + G::OFF_C + s * G::C_BYTES;
       mbar_expect_tx(bar, G::C_BYTES);
-      tma_load_4d(smem_u32(dst), &maps.c9, tx0, ty0, k, 0, bar);
-      tma_load_4d(smem_u32(dst + 9 * NTHR * G::ES), &maps.c3, tx0, ty0, k, 10, bar);
+      load_coefs<VT>(maps, smem_u32(dst), NTHR * G::ES, tx0, ty0, k, bar);
     };
     auto issue_m = [&](int o) {
       const unsigned f = fm0 + o, s = f % NM;
@@ -558,8 +631,8 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
       mbar_expect_tx(bar, m_bytes);
       if (need_m) tma_load_4d(smem_u32(dst), &maps.m, tx0, ty0, k, 0, bar);
       if (need_t)
-        tma_load_4d(smem_u32(dst + 9 * NTHR * G::ES), tsel == kTsOld ? &maps.x : &maps.t, tx0, ty0,
-                    k, 0, bar);
+        tma_load_4d(smem_u32(dst + G::T_AT * NTHR * G::ES), tsel == kTsOld ? &maps.x : &maps.t,
+                    tx0, ty0, k, 0, bar);
     };
     if (tid == 0) {
       for (int n = 0; n < NW - 1 && n < nplanes; ++n) issue_w(n);
@@ -664,15 +737,23 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
         else
           xy = (const S *)(smem + ((fw0 + n + NW - 1) % NW) * G::W_BYTES);
         const S *cf = (const S *)(smem + G::OFF_C + ((fc0 + o) % NC) * G::C_BYTES);
+        // (VT: mx[0] and my[1] are the only metrics of their rows)
         float mx[3], my[3], mz[3];
+        constexpr int CZ = VT ? 2 : 6, CM = G::CF - 3;
+        if constexpr (VT) {
+          mx[0] = ldv(cf + cidx);
+          my[1] = ldv(cf + NTHR + cidx);
+        } else {
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          mx[q] = ldv(cf + q * NTHR + cidx);
-          my[q] = ldv(cf + (3 + q) * NTHR + cidx);
-          mz[q] = ldv(cf + (6 + q) * NTHR + cidx);
+          for (int q = 0; q < 3; ++q) {
+            mx[q] = ldv(cf + q * NTHR + cidx);
+            my[q] = ldv(cf + (3 + q) * NTHR + cidx);
+          }
         }
-        const float mu = ldv(cf + 9 * NTHR + cidx), lam = ldv(cf + 10 * NTHR + cidx);
-        const float bu = ldv(cf + 11 * NTHR + cidx) * (float)CRHO_OF<S>::v;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) mz[q] = ldv(cf + (CZ + q) * NTHR + cidx);
+        const float mu = ldv(cf + CM * NTHR + cidx), lam = ldv(cf + (CM + 1) * NTHR + cidx);
+        const float bu = ldv(cf + (CM + 2) * NTHR + cidx) * (float)CRHO_OF<S>::v;
         const float bzd = bz_cur * DT * gz;
         float h[9], Lr[9], E[9];
         ElasticSum es;
@@ -687,48 +768,64 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
         // stencil sums, the increment and the RK combination.  The centre
         // tap of the x and y stencils, plane k at this point, is window slot
         // P1 (loaded from the same shared-memory plane one iteration ago).
-        // x direction
-#pragma unroll
-        for (int v = 0; v < 8; v += 2) {
-          const XT *r0 = xy + (v * BY + ys) * BX + xs, *r1 = r0 + BY * BX;
-          const float2 s = stencil2(pk(ldv(r0 - FB1), ldv(r1 - FB1)), pk(win[v][P1], win[v + 1][P1]),
-                                    pk(ldv(r0 + FB1), ldv(r1 + FB1)),
-                                    pk(ldv(r0 + 2 * FB1), ldv(r1 + 2 * FB1)),
-                                    pk(ldv(r0 + 3 * FB1), ldv(r1 + 3 * FB1)));
-          Lr[v] = s.x;
-          Lr[v + 1] = s.y;
-        }
-        {
+        // taps of fields va and vb along stride dst
+        auto two = [&](int va, int vb, int dst) {
+          const XT *r0 = xy + (va * BY + ys) * BX + xs, *r1 = xy + (vb * BY + ys) * BX + xs;
+          const float2 q = stencil2(pk(ldv(r0 - dst), ldv(r1 - dst)), pk(win[va][P1], win[vb][P1]),
+                                    pk(ldv(r0 + dst), ldv(r1 + dst)),
+                                    pk(ldv(r0 + 2 * dst), ldv(r1 + 2 * dst)),
+                                    pk(ldv(r0 + 3 * dst), ldv(r1 + 3 * dst)));
+          Lr[va] = q.x;
+          Lr[vb] = q.y;
+        };
+        auto last = [&](int dst) {
           const XT *r0 = xy + (8 * BY + ys) * BX + xs;
-          Lr[8] = stencil1(ldv(r0 - FB1), win[8][P1], ldv(r0 + FB1), ldv(r0 + 2 * FB1), ldv(r0 + 3 * FB1));
+          Lr[8] = stencil1(ldv(r0 - dst), win[8][P1], ldv(r0 + dst), ldv(r0 + 2 * dst),
+                           ldv(r0 + 3 * dst));
+        };
+        // x direction (VT: the fields that xi_x alone multiplies)
+        if constexpr (VT) {
+          two(0, 1, FB1);
+          two(2, 3, FB1);
+          two(6, 7, FB1);
+          es.add_vert_x(mx[0], bxd, Lr);
+        } else {
+          two(0, 1, FB1);
+          two(2, 3, FB1);
+          two(4, 5, FB1);
+          two(6, 7, FB1);
+          last(FB1);
+          es.template add<true>(mx, bxd, Lr);
         }
-        es.add<true>(mx, bxd, Lr);
         if constexpr (PMLK) {
           if (sx >= 0) {  // profile values d, alpha + d, beta at this x
-            elastic9(mx, Lr, mu, lam, bu, E);
+            if constexpr (VT)
+              elastic9_vert<0>(mx[0], Lr, mu, lam, bu, E);
+            else
+              elastic9(mx, Lr, mu, lam, bu, E);
             pml_apply<RK>(a.slab[sx], slab_pos(a.slab[sx], i, j, k), E, dlx, adx, btx, DT, cB, cA, pc, HP, pin);
           }
         }
         // y direction
-#pragma unroll
-        for (int v = 0; v < 8; v += 2) {
-          const XT *c0 = xy + (v * BY + ys) * BX + xs, *c1 = c0 + BY * BX;
-          const float2 s = stencil2(pk(ldv(c0 - FB2 * BX), ldv(c1 - FB2 * BX)), pk(win[v][P1], win[v + 1][P1]),
-                                    pk(ldv(c0 + FB2 * BX), ldv(c1 + FB2 * BX)),
-                                    pk(ldv(c0 + 2 * FB2 * BX), ldv(c1 + 2 * FB2 * BX)),
-                                    pk(ldv(c0 + 3 * FB2 * BX), ldv(c1 + 3 * FB2 * BX)));
-          Lr[v] = s.x;
-          Lr[v + 1] = s.y;
+        if constexpr (VT) {
+          two(0, 1, FB2 * BX);
+          two(2, 4, FB2 * BX);
+          two(6, 8, FB2 * BX);
+          es.add_vert_y(my[1], byd, Lr);
+        } else {
+          two(0, 1, FB2 * BX);
+          two(2, 3, FB2 * BX);
+          two(4, 5, FB2 * BX);
+          two(6, 7, FB2 * BX);
+          last(FB2 * BX);
+          es.template add<false>(my, byd, Lr);
         }
-        {
-          const XT *c0 = xy + (8 * BY + ys) * BX + xs;
-          Lr[8] = stencil1(ldv(c0 - FB2 * BX), win[8][P1], ldv(c0 + FB2 * BX), ldv(c0 + 2 * FB2 * BX),
-                           ldv(c0 + 3 * FB2 * BX));
-        }
-        es.add<false>(my, byd, Lr);
         if constexpr (PMLK) {
           if (sy >= 0) {
-            elastic9(my, Lr, mu, lam, bu, E);
+            if constexpr (VT)
+              elastic9_vert<1>(my[1], Lr, mu, lam, bu, E);
+            else
+              elastic9(my, Lr, mu, lam, bu, E);
             pml_apply<RK>(a.slab[sy], slab_pos(a.slab[sy], i, j, k), E, dly, ady, bty, DT, cB, cA, pc,
                           sh == sy ? HP : 0, pin);
           }
@@ -743,7 +840,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
           Lr[v + 1] = s.y;
         }
         Lr[8] = stencil1(win[8][P0], win[8][P1], win[8][P2], win[8][P3], win[8][P4]);
-        es.add<false>(mz, bzd, Lr);
+        es.template add<false>(mz, bzd, Lr);
         const bool zslab = PMLK && a.nslab && k < HALO + a.npml;
         if constexpr (PMLK) {
           if (zslab) {
@@ -765,7 +862,7 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
         // stages 1-2: t += B h, out = m + A h; stage 3: out = t + B4 h;
         // in a whole step only stage 2 writes t, see StageArgs::lean
         const S *ms = (const S *)(smem + G::OFF_M + ((fm0 + o) % NM) * G::M_BYTES);
-        const S *ts = ms + 9 * NTHR;
+        const S *ts = ms + G::T_AT * NTHR;
         const long long ctr = L.at(i, j, k);
         const float cT = ST == 0 ? kB1 : ST == 1 ? cB : 0.0f;
         const float cO = ST == 0 ? kA2rk : ST == 1 ? cA : kB4;
@@ -857,17 +954,17 @@ __device__ __forceinline__ void stream_body(const Src &src, int *err) {
   if (tid == 0) queue_leave(src.counter());
 }
 
-template <typename S, int TYv, int FB1, int FB2, int FB3, bool PMLK, int RK>
+template <typename S, int TYv, int FB1, int FB2, int FB3, bool PMLK, int RK, bool VT>
 __global__ void __launch_bounds__(TX * TYv, Geo<S, TYv>::MINB)
     stage_stream_kernel(const __grid_constant__ Maps maps, const __grid_constant__ StageArgs<S> a,
                         const __grid_constant__ Work wk, int *err) {
-  stream_body<S, TYv, FB1, FB2, FB3, PMLK, RK>(SingleSrc<S>{maps, a, wk}, err);
+  stream_body<S, TYv, FB1, FB2, FB3, PMLK, RK, VT>(SingleSrc<S>{maps, a, wk}, err);
 }
 
-template <typename S, int FB1, int FB2, int FB3, bool PMLK, int RK>
+template <typename S, int FB1, int FB2, int FB3, bool PMLK, int RK, bool VT>
 __global__ void __launch_bounds__(TX * 16, 1)
     stage_stream_batch_kernel(const __grid_constant__ BatchParams<S> p, int *err) {
-  stream_body<S, 16, FB1, FB2, FB3, PMLK, RK>(BatchSrc<S>{p}, err);
+  stream_body<S, 16, FB1, FB2, FB3, PMLK, RK, VT>(BatchSrc<S>{p}, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -887,11 +984,12 @@ __global__ void __launch_bounds__(TX * 16, 1)
 // copy of each plane, converted once cooperatively, measured slower: the
 // extra barrier-bound work per plane and the shallower W ring cost more
 // than the conversions it saves.)
-template <typename S> struct PairGeo {
+template <typename S, int RK = 0, bool VT = false> struct PairGeo {
   static constexpr int TY = 8, TXP = 64, NTHR = 256, PLANE = TY * TXP;
   static constexpr int BY = TY + 4, BX = 8 + TXP + 8;
   static constexpr int W_BYTES = ((9 * BY * BX * 2) + 127) / 128 * 128;
-  static constexpr int C_BYTES = 12 * PLANE * 2;
+  static constexpr int CF = VT ? 8 : 12;
+  static constexpr int C_BYTES = CF * PLANE * 2;
   static constexpr int M_BYTES = 18 * PLANE * 2;
   static constexpr int NW = 4, NC = 3, NM = 3;
   static constexpr int OFF_C = NW * W_BYTES;
@@ -932,6 +1030,26 @@ struct ElasticSum2 {
     s7 = f2fma(a0, L[2], FIRST ? f2mul(a2, L[0]) : f2fma(a2, L[0], s7));
     s8 = f2fma(a1, L[2], FIRST ? f2mul(a2, L[1]) : f2fma(a2, L[1], s8));
   }
+  __device__ __forceinline__ void add_vert_x(float2 m, float2 g, const float2 L[9]) {
+    const float2 a = f2mul(g, m);
+    v0 = f2mul(a, L[3]);
+    v1 = f2mul(a, L[6]);
+    v2 = f2mul(a, L[7]);
+    nx = f2mul(a, L[0]);
+    ny = nz = pk(0.0f);
+    s6 = f2mul(a, L[1]);
+    s7 = f2mul(a, L[2]);
+    s8 = pk(0.0f);
+  }
+  __device__ __forceinline__ void add_vert_y(float2 m, float2 g, const float2 L[9]) {
+    const float2 a = f2mul(g, m);
+    v0 = f2fma(a, L[6], v0);
+    v1 = f2fma(a, L[4], v1);
+    v2 = f2fma(a, L[8], v2);
+    ny = f2mul(a, L[1]);
+    s6 = f2fma(a, L[0], s6);
+    s8 = f2mul(a, L[2]);
+  }
   __device__ __forceinline__ void finish(float2 mu, float2 lam, float2 b, float2 h[9]) const {
     h[0] = f2mul(v0, b);
     h[1] = f2mul(v1, b);
@@ -959,11 +1077,11 @@ __device__ __forceinline__ void item_of_pair(const Work &w, int item, int &pxi, 
   ke = min(kb + w.chunk_i, kend);
 }
 
-template <typename S, int FB1, int FB2, int FB3, int RK>
+template <typename S, int FB1, int FB2, int FB3, int RK, bool VT>
 __global__ void __launch_bounds__(256, 1)
     stage_pair_kernel(const __grid_constant__ Maps maps, const __grid_constant__ StageArgs<S> a,
                       const __grid_constant__ Work wk, int *err) {
-  using G = PairGeo<S>;
+  using G = PairGeo<S, RK, VT>;
   constexpr int TY = G::TY, PLANE = G::PLANE, BY = G::BY, BX = G::BX, NTHR = G::NTHR;
   constexpr int NW = G::NW, NC = G::NC, NM = G::NM;
   constexpr int DIR = -FB3;  // sweep direction in z
@@ -1027,8 +1145,7 @@ __global__ void __launch_bounds__(256, 1)
       const uint32_t bar = smem_u32(&bc[q]);
       unsigned char *dst = smem + G::OFF_C + q * G::C_BYTES;
       mbar_expect_tx(bar, G::C_BYTES);
-      tma_load_4d(smem_u32(dst), &maps.c9, tx0, ty0, k, 0, bar);
-      tma_load_4d(smem_u32(dst + 9 * PLANE * 2), &maps.c3, tx0, ty0, k, 10, bar);
+      load_coefs<VT>(maps, smem_u32(dst), PLANE * 2, tx0, ty0, k, bar);
     };
     auto issue_m = [&](int o) {
       const unsigned f = fm0 + o, q = f % NM;
@@ -1087,14 +1204,21 @@ __global__ void __launch_bounds__(256, 1)
         const S *xy = (const S *)(smem + ((fw0 + n + NW - 1) % NW) * G::W_BYTES);  // plane k
         const S *cf = (const S *)(smem + G::OFF_C + ((fc0 + o) % NC) * G::C_BYTES);
         float2 mx[3], my[3], mz[3];
+        constexpr int CZ = VT ? 2 : 6, CM = G::CF - 3;
+        if constexpr (VT) {
+          mx[0] = ld2(cf + cidx);
+          my[1] = ld2(cf + PLANE + cidx);
+        } else {
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          mx[q] = ld2(cf + q * PLANE + cidx);
-          my[q] = ld2(cf + (3 + q) * PLANE + cidx);
-          mz[q] = ld2(cf + (6 + q) * PLANE + cidx);
+          for (int q = 0; q < 3; ++q) {
+            mx[q] = ld2(cf + q * PLANE + cidx);
+            my[q] = ld2(cf + (3 + q) * PLANE + cidx);
+          }
         }
-        const float2 mu = ld2(cf + 9 * PLANE + cidx), lam = ld2(cf + 10 * PLANE + cidx);
-        const float2 bu = f2mul(ld2(cf + 11 * PLANE + cidx), pk((float)CRHO_OF<S>::v));
+#pragma unroll
+        for (int q = 0; q < 3; ++q) mz[q] = ld2(cf + (CZ + q) * PLANE + cidx);
+        const float2 mu = ld2(cf + CM * PLANE + cidx), lam = ld2(cf + (CM + 1) * PLANE + cidx);
+        const float2 bu = f2mul(ld2(cf + (CM + 2) * PLANE + cidx), pk((float)CRHO_OF<S>::v));
         const float2 bzd = pk(bz_cur * DT * gz);
         float2 h[9], Lr[9];
         ElasticSum2 es;
@@ -1102,6 +1226,7 @@ __global__ void __launch_bounds__(256, 1)
         // pair (plane k at i, i + 1) is window slot P1
 #pragma unroll
         for (int v = 0; v < 9; ++v) {
+          if (VT && (v == 4 || v == 5 || v == 8)) continue;  // no xi_x term
           const S *row = xy + (v * BY + ys) * BX + xs;
           const float2 cen = win[v][P1];
           if (FB1 > 0) {
@@ -1116,20 +1241,27 @@ __global__ void __launch_bounds__(256, 1)
                              make_float2(xm3, w21.x));
           }
         }
-        es.add<true>(mx, bxd, Lr);
+        if constexpr (VT)
+          es.add_vert_x(mx[0], bxd, Lr);
+        else
+          es.template add<true>(mx, bxd, Lr);
         // y direction
 #pragma unroll
         for (int v = 0; v < 9; ++v) {
+          if (VT && (v == 3 || v == 5 || v == 7)) continue;  // no eta_y term
           const S *c0 = xy + (v * BY + ys) * BX + xs;
           Lr[v] = stencil2(ld2(c0 - FB2 * BX), win[v][P1], ld2(c0 + FB2 * BX),
                            ld2(c0 + 2 * FB2 * BX), ld2(c0 + 3 * FB2 * BX));
         }
-        es.add<false>(my, byd, Lr);
+        if constexpr (VT)
+          es.add_vert_y(my[1], byd, Lr);
+        else
+          es.template add<false>(my, byd, Lr);
         // z direction: W[k - m*DIR] for m = -1..3 sits in slots P0 (q = k + DIR) .. P4
 #pragma unroll
         for (int v = 0; v < 9; ++v)
           Lr[v] = stencil2(win[v][P0], win[v][P1], win[v][P2], win[v][P3], win[v][P4]);
-        es.add<false>(mz, bzd, Lr);
+        es.template add<false>(mz, bzd, Lr);
         es.finish(mu, lam, bu, h);
         // RK4 combination (wave_rk.cpp:13-99), as the one-point kernel
         const S *ms = (const S *)(smem + G::OFF_M + ((fm0 + o) % NM) * G::M_BYTES);
@@ -1216,12 +1348,12 @@ cudaError_t ensure_smem_attr(K kern, int smem, std::atomic<unsigned long long> &
   return e;
 }
 
-template <typename S, int TYv, int FB1, int FB2, int FB3, bool PMLK, int RK>
+template <typename S, int TYv, int FB1, int FB2, int FB3, bool PMLK, int RK, bool VT>
 cudaError_t launch_variant(const StageArgs<S> &a, const Maps &maps, const Work &wk, int *err,
                            int nsm, cudaStream_t st) {
-  using G = Geo<S, TYv, PMLK>;
+  using G = Rings<S, TYv, PMLK, RK, VT>;
   static std::atomic<unsigned long long> attr_done{0};
-  auto kern = stage_stream_kernel<S, TYv, FB1, FB2, FB3, PMLK, RK>;
+  auto kern = stage_stream_kernel<S, TYv, FB1, FB2, FB3, PMLK, RK, VT>;
   const int smem = G::SMEM;
   cudaError_t e = ensure_smem_attr(kern, smem, attr_done);
   if (e != cudaSuccess) return e;
@@ -1311,7 +1443,7 @@ WorkPlan plan_work(const StageArgs<S> &a, int nsm, int *counter, int group_tiles
 
 // Splits the stage into the interior launch (tiles and chunks that touch no
 // PML slab) and the PML launch (the rest), see Work.
-template <typename S, int TYv, int FB1, int FB2, int FB3, int RK>
+template <typename S, int TYv, int FB1, int FB2, int FB3, int RK, bool VT>
 cudaError_t launch_one(const StageArgs<S> &a, const Maps &maps, int *err, int *counter,
                        StreamPair st, int *nlaunch) {
   const int nsm = sm_count();
@@ -1320,7 +1452,7 @@ cudaError_t launch_one(const StageArgs<S> &a, const Maps &maps, int *err, int *c
   Work wi = wp.wk;
   wi.nitems = wp.n_in;
   if (wi.nitems > 0) {
-    e = launch_variant<S, TYv, FB1, FB2, FB3, false, RK>(a, maps, wi, err, nsm, st.main);
+    e = launch_variant<S, TYv, FB1, FB2, FB3, false, RK, VT>(a, maps, wi, err, nsm, st.main);
     if (e != cudaSuccess) return e;
     if (nlaunch) ++*nlaunch;
   }
@@ -1328,7 +1460,7 @@ cudaError_t launch_one(const StageArgs<S> &a, const Maps &maps, int *err, int *c
   wq.nitems = wp.n_pml;
   wq.counter = counter + 2;
   if (wq.nitems > 0) {
-    e = launch_variant<S, TYv, FB1, FB2, FB3, true, RK>(a, maps, wq, err, nsm, st.pml);
+    e = launch_variant<S, TYv, FB1, FB2, FB3, true, RK, VT>(a, maps, wq, err, nsm, st.pml);
     if (e != cudaSuccess) return e;
     if (nlaunch) ++*nlaunch;
   }
@@ -1340,7 +1472,7 @@ cudaError_t launch_one(const StageArgs<S> &a, const Maps &maps, int *err, int *c
 // inside the grid) and the one-point 32 x 8 PML variant for every other
 // tile and chunk (an odd interior tile column and partial edge tiles
 // included).  16-bit storage only.
-template <typename S, int FB1, int FB2, int FB3, int RK>
+template <typename S, int FB1, int FB2, int FB3, int RK, bool VT>
 cudaError_t launch_one_pair(const StageArgs<S> &a, const Maps &m8, const Maps &mp, int *err,
                             int *counter, StreamPair st, int *nlaunch) {
   if constexpr (sizeof(S) != 2) {
@@ -1364,9 +1496,9 @@ cudaError_t launch_one_pair(const StageArgs<S> &a, const Maps &m8, const Maps &m
     Work wi = w;
     wi.nitems = tiles_in / 2 * w.nic;
     if (wi.nitems > 0) {
-      using G = PairGeo<S>;
+      using G = PairGeo<S, RK, VT>;
       static std::atomic<unsigned long long> attr_done{0};
-      auto kern = stage_pair_kernel<S, FB1, FB2, FB3, RK>;
+      auto kern = stage_pair_kernel<S, FB1, FB2, FB3, RK, VT>;
       e = ensure_smem_attr(kern, G::SMEM, attr_done);
       if (e != cudaSuccess) return e;
       kern<<<std::min(wi.nitems, nsm), G::NTHR, G::SMEM, st.main>>>(mp, a, wi, err);
@@ -1378,7 +1510,7 @@ cudaError_t launch_one_pair(const StageArgs<S> &a, const Maps &m8, const Maps &m
     wq.nitems = w.nzc * tiles + (tiles - tiles_in) * w.nic;
     wq.counter = counter + 2;
     if (wq.nitems > 0) {
-      e = launch_variant<S, 8, FB1, FB2, FB3, true, RK>(a, m8, wq, err, nsm, st.pml);
+      e = launch_variant<S, 8, FB1, FB2, FB3, true, RK, VT>(a, m8, wq, err, nsm, st.pml);
       if (e != cudaSuccess) return e;
       if (nlaunch) ++*nlaunch;
     }
@@ -1386,13 +1518,13 @@ cudaError_t launch_one_pair(const StageArgs<S> &a, const Maps &m8, const Maps &m
   }
 }
 
-template <typename S, int FB1, int FB2, int FB3, bool PMLK, int RK>
+template <typename S, int FB1, int FB2, int FB3, bool PMLK, int RK, bool VT>
 cudaError_t launch_batch_variant(const BatchParams<S> &p, int items, int *err, int nsm,
                                  cudaStream_t st) {
-  using G = Geo<S, 16, PMLK>;
+  using G = Rings<S, 16, PMLK, RK, VT>;
   static_assert(sizeof(BatchParams<S>) <= 32000, "kernel parameter space");
   static std::atomic<unsigned long long> attr_done{0};
-  auto kern = stage_stream_batch_kernel<S, FB1, FB2, FB3, PMLK, RK>;
+  auto kern = stage_stream_batch_kernel<S, FB1, FB2, FB3, PMLK, RK, VT>;
   const int smem = G::SMEM;
   cudaError_t e = ensure_smem_attr(kern, smem, attr_done);
   if (e != cudaSuccess) return e;
@@ -1402,7 +1534,7 @@ cudaError_t launch_batch_variant(const BatchParams<S> &p, int items, int *err, i
 
 // One stage of n scenarios that share the MacCormack signs: kBatchMax
 // scenarios per launch pair (interior items of all of them, then PML items).
-template <typename S, int FB1, int FB2, int FB3, int RK>
+template <typename S, int FB1, int FB2, int FB3, int RK, bool VT>
 cudaError_t launch_batch(const StageArgs<S> *args, const void *const *maps, int n, int *err,
                          int *counter, StreamPair st, int *nlaunch) {
   const int nsm = sm_count();
@@ -1438,8 +1570,8 @@ cudaError_t launch_batch(const StageArgs<S> *args, const void *const *maps, int 
       bp->n = m;
       bp->counter = counter + 2 * pass;
       cudaError_t e = pass == 0
-                          ? launch_batch_variant<S, FB1, FB2, FB3, false, RK>(*bp, total, err, nsm, st.main)
-                          : launch_batch_variant<S, FB1, FB2, FB3, true, RK>(*bp, total, err, nsm, st.pml);
+                          ? launch_batch_variant<S, FB1, FB2, FB3, false, RK, VT>(*bp, total, err, nsm, st.main)
+                          : launch_batch_variant<S, FB1, FB2, FB3, true, RK, VT>(*bp, total, err, nsm, st.pml);
       if (e != cudaSuccess) return e;
       if (nlaunch) ++*nlaunch;
     }
@@ -1519,6 +1651,7 @@ int encode_stream_maps(const S *wave, const S *cjm, const S *wm, const S *t, con
     if (!rc) rc = encode_map<S>(wave, L, 9, Geo<S, 16>::BX, ty + 4, 9, &m.w);
     if (!rc) rc = encode_map<S>(cjm, L, 13, TX, ty, 9, &m.c9);
     if (!rc) rc = encode_map<S>(cjm, L, 13, TX, ty, 3, &m.c3);
+    if (!rc) rc = encode_map<S>(cjm, L, 13, TX, ty, 1, &m.c1);
     if (!rc) rc = encode_map<S>(wm, L, 9, TX, ty, 9, &m.m);
     if (!rc) rc = encode_map<S>(t, L, 9, TX, ty, 9, &m.t);
     if (!rc) rc = encode_map<S>(x, L, 9, TX, ty, 9, &m.x);
@@ -1529,6 +1662,7 @@ int encode_stream_maps(const S *wave, const S *cjm, const S *wm, const S *t, con
     if (!rc) rc = encode_map<S>(wave, L, 9, G::BX, G::BY, 9, &m.w);
     if (!rc) rc = encode_map<S>(cjm, L, 13, G::TXP, G::TY, 9, &m.c9);
     if (!rc) rc = encode_map<S>(cjm, L, 13, G::TXP, G::TY, 3, &m.c3);
+    if (!rc) rc = encode_map<S>(cjm, L, 13, G::TXP, G::TY, 1, &m.c1);
     if (!rc) rc = encode_map<S>(wm, L, 9, G::TXP, G::TY, 9, &m.m);
     if (!rc) rc = encode_map<S>(t, L, 9, G::TXP, G::TY, 9, &m.t);
     if (!rc) rc = encode_map<S>(x, L, 9, G::TXP, G::TY, 9, &m.x);
@@ -1542,83 +1676,106 @@ inline int rk_class(int irk, int lean) {
   return irk == 3 ? 3 : lean ? 4 + irk : irk == 0 ? 0 : 1;
 }
 
-template <typename S, int TYv, int RK>
+template <typename S, int TYv, int RK, bool VT>
 cudaError_t launch_fb_rk(const StageArgs<S> &a, const Maps &m, int *err, int *counter,
                          StreamPair st, int *nlaunch) {
   const int code = (a.fb1 > 0) * 4 + (a.fb2 > 0) * 2 + (a.fb3 > 0);
   switch (code) {
-    case 0: return launch_one<S, TYv, -1, -1, -1, RK>(a, m, err, counter, st, nlaunch);
-    case 1: return launch_one<S, TYv, -1, -1, 1, RK>(a, m, err, counter, st, nlaunch);
-    case 2: return launch_one<S, TYv, -1, 1, -1, RK>(a, m, err, counter, st, nlaunch);
-    case 3: return launch_one<S, TYv, -1, 1, 1, RK>(a, m, err, counter, st, nlaunch);
-    case 4: return launch_one<S, TYv, 1, -1, -1, RK>(a, m, err, counter, st, nlaunch);
-    case 5: return launch_one<S, TYv, 1, -1, 1, RK>(a, m, err, counter, st, nlaunch);
-    case 6: return launch_one<S, TYv, 1, 1, -1, RK>(a, m, err, counter, st, nlaunch);
-    default: return launch_one<S, TYv, 1, 1, 1, RK>(a, m, err, counter, st, nlaunch);
+    case 0: return launch_one<S, TYv, -1, -1, -1, RK, VT>(a, m, err, counter, st, nlaunch);
+    case 1: return launch_one<S, TYv, -1, -1, 1, RK, VT>(a, m, err, counter, st, nlaunch);
+    case 2: return launch_one<S, TYv, -1, 1, -1, RK, VT>(a, m, err, counter, st, nlaunch);
+    case 3: return launch_one<S, TYv, -1, 1, 1, RK, VT>(a, m, err, counter, st, nlaunch);
+    case 4: return launch_one<S, TYv, 1, -1, -1, RK, VT>(a, m, err, counter, st, nlaunch);
+    case 5: return launch_one<S, TYv, 1, -1, 1, RK, VT>(a, m, err, counter, st, nlaunch);
+    case 6: return launch_one<S, TYv, 1, 1, -1, RK, VT>(a, m, err, counter, st, nlaunch);
+    default: return launch_one<S, TYv, 1, 1, 1, RK, VT>(a, m, err, counter, st, nlaunch);
   }
 }
-template <typename S, int RK>
+template <typename S, int RK, bool VT>
 cudaError_t launch_fb_rk_pair(const StageArgs<S> &a, const MapSet &ms, int *err, int *counter,
                               StreamPair st, int *nlaunch) {
   const Maps &m8 = ms.ty8, &mp = ms.pair;
   switch ((a.fb1 > 0) * 4 + (a.fb2 > 0) * 2 + (a.fb3 > 0)) {
-    case 0: return launch_one_pair<S, -1, -1, -1, RK>(a, m8, mp, err, counter, st, nlaunch);
-    case 1: return launch_one_pair<S, -1, -1, 1, RK>(a, m8, mp, err, counter, st, nlaunch);
-    case 2: return launch_one_pair<S, -1, 1, -1, RK>(a, m8, mp, err, counter, st, nlaunch);
-    case 3: return launch_one_pair<S, -1, 1, 1, RK>(a, m8, mp, err, counter, st, nlaunch);
-    case 4: return launch_one_pair<S, 1, -1, -1, RK>(a, m8, mp, err, counter, st, nlaunch);
-    case 5: return launch_one_pair<S, 1, -1, 1, RK>(a, m8, mp, err, counter, st, nlaunch);
-    case 6: return launch_one_pair<S, 1, 1, -1, RK>(a, m8, mp, err, counter, st, nlaunch);
-    default: return launch_one_pair<S, 1, 1, 1, RK>(a, m8, mp, err, counter, st, nlaunch);
+    case 0: return launch_one_pair<S, -1, -1, -1, RK, VT>(a, m8, mp, err, counter, st, nlaunch);
+    case 1: return launch_one_pair<S, -1, -1, 1, RK, VT>(a, m8, mp, err, counter, st, nlaunch);
+    case 2: return launch_one_pair<S, -1, 1, -1, RK, VT>(a, m8, mp, err, counter, st, nlaunch);
+    case 3: return launch_one_pair<S, -1, 1, 1, RK, VT>(a, m8, mp, err, counter, st, nlaunch);
+    case 4: return launch_one_pair<S, 1, -1, -1, RK, VT>(a, m8, mp, err, counter, st, nlaunch);
+    case 5: return launch_one_pair<S, 1, -1, 1, RK, VT>(a, m8, mp, err, counter, st, nlaunch);
+    case 6: return launch_one_pair<S, 1, 1, -1, RK, VT>(a, m8, mp, err, counter, st, nlaunch);
+    default: return launch_one_pair<S, 1, 1, 1, RK, VT>(a, m8, mp, err, counter, st, nlaunch);
   }
 }
 // One stage class of one scenario at the tile forms other than 32 x 16, and
 // of a batch at 32 x 16; instantiated in several translation units per
 // storage type, STREAM_PART of them (the classes of a part are listed at
 // STREAM_INSTANTIATE).
-template <typename S, int RK>
+template <typename S, int RK, bool VT>
 cudaError_t launch_single_rk(const StageArgs<S> &a, const void *maps, int *err, int *counter,
                              StreamPair st, int *nlaunch, int tile_rows) {
   const MapSet &ms = *(const MapSet *)maps;
-  if (tile_rows == 8) return launch_fb_rk<S, 8, RK>(a, ms.ty8, err, counter, st, nlaunch);
+  if (tile_rows == 8) return launch_fb_rk<S, 8, RK, VT>(a, ms.ty8, err, counter, st, nlaunch);
   if constexpr (sizeof(S) == 2) {
-    if (tile_rows == kTilePair) return launch_fb_rk_pair<S, RK>(a, ms, err, counter, st, nlaunch);
+    if (tile_rows == kTilePair) return launch_fb_rk_pair<S, RK, VT>(a, ms, err, counter, st, nlaunch);
   }
   return cudaErrorInvalidValue;
 }
-template <typename S, int RK>
+template <typename S, int RK, bool VT>
 cudaError_t launch_batch_rk(const StageArgs<S> *args, const void *const *maps, int n, int *err,
                             int *counter, StreamPair st, int *nlaunch) {
   const StageArgs<S> &a = args[0];
   switch ((a.fb1 > 0) * 4 + (a.fb2 > 0) * 2 + (a.fb3 > 0)) {
-    case 0: return launch_batch<S, -1, -1, -1, RK>(args, maps, n, err, counter, st, nlaunch);
-    case 1: return launch_batch<S, -1, -1, 1, RK>(args, maps, n, err, counter, st, nlaunch);
-    case 2: return launch_batch<S, -1, 1, -1, RK>(args, maps, n, err, counter, st, nlaunch);
-    case 3: return launch_batch<S, -1, 1, 1, RK>(args, maps, n, err, counter, st, nlaunch);
-    case 4: return launch_batch<S, 1, -1, -1, RK>(args, maps, n, err, counter, st, nlaunch);
-    case 5: return launch_batch<S, 1, -1, 1, RK>(args, maps, n, err, counter, st, nlaunch);
-    case 6: return launch_batch<S, 1, 1, -1, RK>(args, maps, n, err, counter, st, nlaunch);
-    default: return launch_batch<S, 1, 1, 1, RK>(args, maps, n, err, counter, st, nlaunch);
+    case 0: return launch_batch<S, -1, -1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+    case 1: return launch_batch<S, -1, -1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+    case 2: return launch_batch<S, -1, 1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+    case 3: return launch_batch<S, -1, 1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+    case 4: return launch_batch<S, 1, -1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+    case 5: return launch_batch<S, 1, -1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+    case 6: return launch_batch<S, 1, 1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+    default: return launch_batch<S, 1, 1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
   }
 }
 
-#define STREAM_CLASS(EXT, S, RK)                                                                  \
-  EXT template cudaError_t launch_single_rk<S, RK>(const StageArgs<S> &, const void *, int *,     \
-                                                   int *, StreamPair, int *, int);                \
-  EXT template cudaError_t launch_batch_rk<S, RK>(const StageArgs<S> *, const void *const *, int, \
-                                                  int *, int *, StreamPair, int *);
-// The classes of a storage type over three translation units: part 0 the
-// single-stage forms and the dispatch, parts 1 and 2 whole steps.
+#define STREAM_CLASS(EXT, S, RK, VT)                                                              \
+  EXT template cudaError_t launch_single_rk<S, RK, VT>(const StageArgs<S> &, const void *, int *, \
+                                                       int *, StreamPair, int *, int);            \
+  EXT template cudaError_t launch_batch_rk<S, RK, VT>(const StageArgs<S> *, const void *const *,  \
+                                                      int, int *, int *, StreamPair, int *);
+// The classes of a storage type over translation units: part 0 the
+// single-stage forms and the dispatch, parts 1 and 2 whole steps, parts 3 and
+// 4 whole steps on vertically stretched grids.
 #if STREAM_PART == 0
-#define STREAM_INSTANTIATE(S)                                                            \
-  STREAM_CLASS(, S, 0) STREAM_CLASS(, S, 1)                                              \
-  STREAM_CLASS(extern, S, 3) STREAM_CLASS(extern, S, 4) STREAM_CLASS(extern, S, 5)       \
-  STREAM_CLASS(extern, S, 6)
-#elif STREAM_PART == 1
-#define STREAM_INSTANTIATE(S) STREAM_CLASS(, S, 3) STREAM_CLASS(, S, 4)
+#define STREAM_INSTANTIATE(S)                                                               \
+  STREAM_CLASS(, S, 0, false) STREAM_CLASS(, S, 1, false)                                   \
+  STREAM_CLASS(extern, S, 3, false) STREAM_CLASS(extern, S, 4, false)                       \
+  STREAM_CLASS(extern, S, 5, false) STREAM_CLASS(extern, S, 6, false)                       \
+  STREAM_CLASS(extern, S, 3, true) STREAM_CLASS(extern, S, 4, true)                         \
+  STREAM_CLASS(extern, S, 5, true) STREAM_CLASS(extern, S, 6, true)
 #else
-#define STREAM_INSTANTIATE(S) STREAM_CLASS(, S, 5) STREAM_CLASS(, S, 6)
+#define STREAM_VT (STREAM_PART > 2)
+#if STREAM_PART % 2
+#define STREAM_INSTANTIATE(S) STREAM_CLASS(, S, 3, STREAM_VT) STREAM_CLASS(, S, 4, STREAM_VT)
+#else
+#define STREAM_INSTANTIATE(S) STREAM_CLASS(, S, 5, STREAM_VT) STREAM_CLASS(, S, 6, STREAM_VT)
 #endif
+#endif
+
+// Calls f with the stage class of a launch as a compile-time constant (the
+// single-stage classes take every grid as a general one).
+template <typename S, typename F> cudaError_t with_class(const StageArgs<S> &a, F f) {
+  using std::integral_constant;
+  auto vt = [&](auto rk) {
+    return a.vert ? f(rk, std::true_type()) : f(rk, std::false_type());
+  };
+  switch (rk_class(a.irk, a.lean)) {
+    case 0: return f(integral_constant<int, 0>(), std::false_type());
+    case 1: return f(integral_constant<int, 1>(), std::false_type());
+    case 3: return vt(integral_constant<int, 3>());
+    case 4: return vt(integral_constant<int, 4>());
+    case 5: return vt(integral_constant<int, 5>());
+    default: return vt(integral_constant<int, 6>());
+  }
+}
 
 template <typename S>
 cudaError_t launch_stage_stream(const StageArgs<S> &a, const void *maps_in, int *err, int *counter,
@@ -1631,14 +1788,10 @@ cudaError_t launch_stage_stream(const StageArgs<S> &a, const void *maps_in, int 
   if (tile_rows == 16) {
     e = launch_stage_stream_batch<S>(&a, &maps_in, 1, err, counter, st, nlaunch);
   } else {
-    switch (rk_class(a.irk, a.lean)) {
-      case 0: e = launch_single_rk<S, 0>(a, maps_in, err, counter, st, nlaunch, tile_rows); break;
-      case 1: e = launch_single_rk<S, 1>(a, maps_in, err, counter, st, nlaunch, tile_rows); break;
-      case 3: e = launch_single_rk<S, 3>(a, maps_in, err, counter, st, nlaunch, tile_rows); break;
-      case 4: e = launch_single_rk<S, 4>(a, maps_in, err, counter, st, nlaunch, tile_rows); break;
-      case 5: e = launch_single_rk<S, 5>(a, maps_in, err, counter, st, nlaunch, tile_rows); break;
-      default: e = launch_single_rk<S, 6>(a, maps_in, err, counter, st, nlaunch, tile_rows);
-    }
+    e = with_class(a, [&](auto rk, auto vt) {
+      return launch_single_rk<S, decltype(rk)::value, decltype(vt)::value>(a, maps_in, err, counter,
+                                                                          st, nlaunch, tile_rows);
+    });
   }
   if (e != cudaSuccess) return e;
   if (after_main) e = cudaEventRecord(after_main, st.main);
@@ -1650,16 +1803,12 @@ cudaError_t launch_stage_stream_batch(const StageArgs<S> *args, const void *cons
   if (n <= 0) return cudaSuccess;
   for (int q = 1; q < n; ++q)
     if (args[q].fb1 != args[0].fb1 || args[q].fb2 != args[0].fb2 || args[q].fb3 != args[0].fb3 ||
-        args[q].irk != args[0].irk || args[q].lean != args[0].lean)
+        args[q].irk != args[0].irk || args[q].lean != args[0].lean || args[q].vert != args[0].vert)
       return cudaErrorInvalidValue;
-  switch (rk_class(args[0].irk, args[0].lean)) {
-    case 0: return launch_batch_rk<S, 0>(args, maps, n, err, counter, st, nlaunch);
-    case 1: return launch_batch_rk<S, 1>(args, maps, n, err, counter, st, nlaunch);
-    case 3: return launch_batch_rk<S, 3>(args, maps, n, err, counter, st, nlaunch);
-    case 4: return launch_batch_rk<S, 4>(args, maps, n, err, counter, st, nlaunch);
-    case 5: return launch_batch_rk<S, 5>(args, maps, n, err, counter, st, nlaunch);
-    default: return launch_batch_rk<S, 6>(args, maps, n, err, counter, st, nlaunch);
-  }
+  return with_class(args[0], [&](auto rk, auto vt) {
+    return launch_batch_rk<S, decltype(rk)::value, decltype(vt)::value>(args, maps, n, err, counter,
+                                                                       st, nlaunch);
+  });
 }
 
 }  // namespace cgfdm
