@@ -129,8 +129,16 @@ __device__ __forceinline__ void rk_apply(const StageArgs<S> &a, R in, R base, R 
   }
 }
 
+// Rows of a 32-column block and the blocks an SM shall hold.  The kernel
+// waits on its loads, so warps in flight count: FP64 compiles to 247 registers
+// by itself, eight warps an SM; three blocks of 128 threads at 168 registers
+// (40 bytes of spills) make it twelve.  FP32 and 16-bit storage need 128.
+template <typename S> struct ExactShape { static constexpr int rows = 8, blocks = 1; };
+template <> struct ExactShape<double> { static constexpr int rows = 4, blocks = 3; };
+
 template <typename S>
-__global__ void __launch_bounds__(256) stage_exact_kernel(StageArgs<S> a) {
+__global__ void __launch_bounds__(32 * ExactShape<S>::rows, ExactShape<S>::blocks)
+    stage_exact_kernel(StageArgs<S> a) {
   using R = typename Arith<S>::R;
   const int i = blockIdx.x * blockDim.x + threadIdx.x + HALO;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + HALO;
@@ -322,11 +330,12 @@ __global__ void __launch_bounds__(256) stage_exact_kernel(StageArgs<S> a) {
 }  // namespace
 
 template <typename S> cudaError_t launch_stage_exact(const StageArgs<S> &a, cudaStream_t st) {
-  // one plane per block: the three free-surface layers of the streaming path
-  // leave no thread idle, and a block's 8 rows share their y-neighbour rows
-  dim3 block(32, 8, 1);
+  // one plane per block, whose rows share their y-neighbour rows
+  constexpr int rows = ExactShape<S>::rows;
+  dim3 block(32, rows, 1);
   if (a.kend <= a.kbeg) return cudaSuccess;
-  dim3 grid((a.L.nx_ - 2 * HALO + 31) / 32, (a.L.ny_ - 2 * HALO + 7) / 8, a.kend - a.kbeg);
+  dim3 grid((a.L.nx_ - 2 * HALO + 31) / 32, (a.L.ny_ - 2 * HALO + rows - 1) / rows,
+            a.kend - a.kbeg);
   stage_exact_kernel<S><<<grid, block, 0, st>>>(a);
   return cudaGetLastError();
 }
