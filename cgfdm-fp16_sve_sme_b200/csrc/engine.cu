@@ -970,7 +970,7 @@ template <typename S> class EngineT : public Engine {
   // stage-1 auxiliary inputs; stage 1 reads those and writes Y and T; the
   // real step rewrites all of them before reading them, so the timing leaves
   // the run unchanged (as stages of a whole step they leave T alone).  Results are cached per (precision, grid).
-  // batch_form: a batch member, which always runs the 32 x 16 form inside
+  // batch_form: a batch member, which always runs the 32 x 8 form inside
   // its batch; only the depth is chosen and the member's own form is kept.
   int tune(cudaStream_t st, bool batch_form = false) {
     const auto key = std::make_tuple((int)d_.precision, d_.nx, d_.ny, d_.nz, d_.npml,
@@ -1000,7 +1000,7 @@ template <typename S> class EngineT : public Engine {
     CUDA_TRY(cudaEventCreate(&e1));
     std::vector<int> forms = {16, 8};
     if (sizeof(S) == 2) forms.push_back(kTilePair);
-    if (batch_form) forms = {16};
+    if (batch_form) forms = {8};
     std::vector<int> chunks = {0, 64, 32};
     if (chunk_fixed_) chunks = {chunk_};
     int best_form = 16, best_chunk = chunks[0];
@@ -1333,7 +1333,7 @@ template <typename S> class BatchT : public BatchBase {
       m->last_stream_ = st;
     }
     if (!tuned_) {
-      // every member's work-item depth for the batch's 32 x 16 form
+      // every member's work-item depth for the batch's 32 x 8 form
       for (auto *m : m_)
         if (m->use_stream_ && !m->chunk_fixed_) {
           int rc = m->tune(st, true);

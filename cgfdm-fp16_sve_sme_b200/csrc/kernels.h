@@ -52,10 +52,10 @@ cudaError_t launch_stage_stream(const StageArgs<S> &a, const void *maps, int *er
                                 int *work_counter, StreamPair st,
                                 cudaEvent_t after_main = nullptr, int *nlaunch = nullptr,
                                 int tile_rows = 16);
-// One stage (same irk and MacCormack signs for all) of n scenarios in
-// persistent launches whose work queue spans all of them (16 scenarios per
-// launch pair); maps[q] is scenario q's encode_stream_maps buffer.  Tile
-// height 16.
+// One stage of a whole step (same irk and MacCormack signs for all) of n
+// scenarios in persistent launches whose work queue spans all of them (16
+// scenarios per launch pair); maps[q] is scenario q's encode_stream_maps
+// buffer.  Tile height 8.
 template <typename S>
 cudaError_t launch_stage_stream_batch(const StageArgs<S> *args, const void *const *maps, int n,
                                       int *err_flag, int *work_counter, StreamPair st,

@@ -502,6 +502,11 @@ template <typename S> struct SingleSrc {
 };
 
 constexpr int kBatchMax = 16;
+// Tile height of a batch's launches: the members are small and middle-sized
+// grids, on which 32 x 8 tiles measured faster than 32 x 16 (161x161x101
+// 0.696 against 0.739 ms a step, 401x401x201 5.24 against 5.49; equal at
+// 601x601x401).
+constexpr int kBatchRows = 8;
 template <typename S> struct BatchParams {
   Maps maps[kBatchMax];
   StageArgs<S> args[kBatchMax];
@@ -962,9 +967,9 @@ __global__ void __launch_bounds__(TX * TYv, Geo<S, TYv>::MINB)
 }
 
 template <typename S, int FB1, int FB2, int FB3, bool PMLK, int RK, bool VT>
-__global__ void __launch_bounds__(TX * 16, 1)
+__global__ void __launch_bounds__(TX * kBatchRows, Geo<S, kBatchRows>::MINB)
     stage_stream_batch_kernel(const __grid_constant__ BatchParams<S> p, int *err) {
-  stream_body<S, 16, FB1, FB2, FB3, PMLK, RK, VT>(BatchSrc<S>{p}, err);
+  stream_body<S, kBatchRows, FB1, FB2, FB3, PMLK, RK, VT>(BatchSrc<S>{p}, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -1521,14 +1526,14 @@ cudaError_t launch_one_pair(const StageArgs<S> &a, const Maps &m8, const Maps &m
 template <typename S, int FB1, int FB2, int FB3, bool PMLK, int RK, bool VT>
 cudaError_t launch_batch_variant(const BatchParams<S> &p, int items, int *err, int nsm,
                                  cudaStream_t st) {
-  using G = Rings<S, 16, PMLK, RK, VT>;
+  using G = Rings<S, kBatchRows, PMLK, RK, VT>;
   static_assert(sizeof(BatchParams<S>) <= 32000, "kernel parameter space");
   static std::atomic<unsigned long long> attr_done{0};
   auto kern = stage_stream_batch_kernel<S, FB1, FB2, FB3, PMLK, RK, VT>;
   const int smem = G::SMEM;
   cudaError_t e = ensure_smem_attr(kern, smem, attr_done);
   if (e != cudaSuccess) return e;
-  kern<<<std::min(items, nsm), G::NTHR, smem, st>>>(p, err);
+  kern<<<std::min(items, nsm * G::MINB), G::NTHR, smem, st>>>(p, err);
   return cudaGetLastError();
 }
 
@@ -1546,7 +1551,7 @@ cudaError_t launch_batch(const StageArgs<S> *args, const void *const *maps, int 
     long long tiles = 0;
     for (int q = 0; q < nb; ++q) {
       const Layout &L = args[b0 + q].L;
-      tiles += (long long)((L.nx_ - 2 * HALO + TX - 1) / TX) * ((L.ny_ - 2 * HALO + 15) / 16);
+      tiles += (long long)((L.nx_ - 2 * HALO + TX - 1) / TX) * ((L.ny_ - 2 * HALO + kBatchRows - 1) / kBatchRows);
     }
     tiles = std::min<long long>(tiles, 1 << 30);
     for (int pass = 0; pass < 2; ++pass) {
@@ -1555,10 +1560,10 @@ cudaError_t launch_batch(const StageArgs<S> *args, const void *const *maps, int 
       for (int q = 0; q < nb; ++q) {
         const StageArgs<S> &a = args[b0 + q];
         if (a.kend <= a.kbeg) continue;
-        const WorkPlan wp = plan_work<S, 16>(a, nsm, counter, (int)tiles);
+        const WorkPlan wp = plan_work<S, kBatchRows>(a, nsm, counter, (int)tiles);
         const int cnt = pass == 0 ? wp.n_in : wp.n_pml;
         if (cnt <= 0) continue;
-        bp->maps[m] = ((const MapSet *)maps[b0 + q])->ty16;
+        bp->maps[m] = ((const MapSet *)maps[b0 + q])->ty8;
         bp->args[m] = a;
         bp->work[m] = wp.wk;
         bp->work[m].nitems = cnt;
@@ -1706,15 +1711,15 @@ cudaError_t launch_fb_rk_pair(const StageArgs<S> &a, const MapSet &ms, int *err,
     default: return launch_one_pair<S, 1, 1, 1, RK, VT>(a, m8, mp, err, counter, st, nlaunch);
   }
 }
-// One stage class of one scenario at the tile forms other than 32 x 16, and
-// of a batch at 32 x 16; instantiated in several translation units per
-// storage type, STREAM_PART of them (the classes of a part are listed at
-// STREAM_INSTANTIATE).
+// One stage class of one scenario and of a batch (whole steps only);
+// instantiated in several translation units per storage type (the classes of
+// a STREAM_PART are listed at STREAM_INSTANTIATE).
 template <typename S, int RK, bool VT>
 cudaError_t launch_single_rk(const StageArgs<S> &a, const void *maps, int *err, int *counter,
                              StreamPair st, int *nlaunch, int tile_rows) {
   const MapSet &ms = *(const MapSet *)maps;
   if (tile_rows == 8) return launch_fb_rk<S, 8, RK, VT>(a, ms.ty8, err, counter, st, nlaunch);
+  if (tile_rows == 16) return launch_fb_rk<S, 16, RK, VT>(a, ms.ty16, err, counter, st, nlaunch);
   if constexpr (sizeof(S) == 2) {
     if (tile_rows == kTilePair) return launch_fb_rk_pair<S, RK, VT>(a, ms, err, counter, st, nlaunch);
   }
@@ -1723,16 +1728,20 @@ cudaError_t launch_single_rk(const StageArgs<S> &a, const void *maps, int *err, 
 template <typename S, int RK, bool VT>
 cudaError_t launch_batch_rk(const StageArgs<S> *args, const void *const *maps, int n, int *err,
                             int *counter, StreamPair st, int *nlaunch) {
-  const StageArgs<S> &a = args[0];
-  switch ((a.fb1 > 0) * 4 + (a.fb2 > 0) * 2 + (a.fb3 > 0)) {
-    case 0: return launch_batch<S, -1, -1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
-    case 1: return launch_batch<S, -1, -1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
-    case 2: return launch_batch<S, -1, 1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
-    case 3: return launch_batch<S, -1, 1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
-    case 4: return launch_batch<S, 1, -1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
-    case 5: return launch_batch<S, 1, -1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
-    case 6: return launch_batch<S, 1, 1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
-    default: return launch_batch<S, 1, 1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+  if constexpr (RK < 3) {
+    return cudaErrorInvalidValue;
+  } else {
+    const StageArgs<S> &a = args[0];
+    switch ((a.fb1 > 0) * 4 + (a.fb2 > 0) * 2 + (a.fb3 > 0)) {
+      case 0: return launch_batch<S, -1, -1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+      case 1: return launch_batch<S, -1, -1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+      case 2: return launch_batch<S, -1, 1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+      case 3: return launch_batch<S, -1, 1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+      case 4: return launch_batch<S, 1, -1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+      case 5: return launch_batch<S, 1, -1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+      case 6: return launch_batch<S, 1, 1, -1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+      default: return launch_batch<S, 1, 1, 1, RK, VT>(args, maps, n, err, counter, st, nlaunch);
+    }
   }
 }
 
@@ -1782,17 +1791,10 @@ cudaError_t launch_stage_stream(const StageArgs<S> &a, const void *maps_in, int 
                                 StreamPair st, cudaEvent_t after_main, int *nlaunch,
                                 int tile_rows) {
   if (a.kend <= a.kbeg) return cudaSuccess;
-  // tile height 16 runs the batched kernel as a batch of one, so that a
-  // scenario gives the same bits alone and inside a batch
-  cudaError_t e;
-  if (tile_rows == 16) {
-    e = launch_stage_stream_batch<S>(&a, &maps_in, 1, err, counter, st, nlaunch);
-  } else {
-    e = with_class(a, [&](auto rk, auto vt) {
-      return launch_single_rk<S, decltype(rk)::value, decltype(vt)::value>(a, maps_in, err, counter,
-                                                                          st, nlaunch, tile_rows);
-    });
-  }
+  cudaError_t e = with_class(a, [&](auto rk, auto vt) {
+    return launch_single_rk<S, decltype(rk)::value, decltype(vt)::value>(a, maps_in, err, counter,
+                                                                        st, nlaunch, tile_rows);
+  });
   if (e != cudaSuccess) return e;
   if (after_main) e = cudaEventRecord(after_main, st.main);
   return e;
