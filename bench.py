@@ -44,11 +44,19 @@ from cgfdm import scenarios as S  # noqa: E402
 REF_EXE = os.path.join(ROOT, "oracle", "_ref", "cgfdm_ref_fp32")
 METRIC = "Gpt-updates/s per RK4 step"
 UNIT = "Gpt-updates/s"
-# Algorithmic HBM bytes per grid point per RK4 step of the fused stage kernels
-# in FP32: per stage 9 stage-input + 12 coefficient reads and 9 output
-# writes; W_n reads in stages 1-2; the RK accumulator written in stage 0,
-# read+written in stages 1-2, read in stage 3 (4 bytes each).
-BYTES_PER_POINT_STEP = {"fp32": 768, "fp64": 1536, "fp16": 384, "bf16": 384}
+# Algorithmic HBM bytes per grid point per RK4 step of the exact-order kernel:
+# per stage 9 stage-input + 12 coefficient reads and 9 output writes; W_n
+# reads in stages 1-2; the RK accumulator written in stage 0, read+written in
+# stages 1-2, read in stage 3.  The streaming kernels' own figure comes from
+# the library's counts (cgfdm_get_kernel_stats), see stream_bytes_per_point.
+EXACT_BYTES_PER_POINT_STEP = {"fp32": 768, "fp64": 1536, "fp16": 384, "bf16": 384}
+
+
+def stream_bytes_per_point(ks, desc):
+    """Algorithmic bytes per point below the free surface and step of the
+    streaming launches of a run."""
+    pts = desc.nx * desc.ny * (desc.nz - 3)
+    return 4.0 * ks["stream_bytes"] / ks["stream_launches"] / pts if ks["stream_launches"] else None
 
 
 def log(*a):
@@ -775,7 +783,7 @@ def main():
         fp16 = {"value": v16, "unit": UNIT, "ms_per_step": ms16_max * 1e3 / args.steps,
                 "speedup_vs_fp32": v16 / value, "tile_form": form16, "chunk_planes": chunk16,
                 "surface_kernel": "tiled" if top16 else "exact-order",
-                "bytes_per_point_step": BYTES_PER_POINT_STEP["fp16"]}
+                "bytes_per_point_step": stream_bytes_per_point(ks16, desc0)}
         if ks16["stream_ms"] > 0:
             a16 = ks16["stream_bytes"] / (ks16["stream_ms"] / 1e3) / 1e9
             pk16 = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))).get("hbm_gbs") \
@@ -812,7 +820,7 @@ def main():
     peak = peaks.get("hbm_gbs")
     peak_src = "measured" if peak else "fallback"
     peak = peak or 6650.0
-    bpp = BYTES_PER_POINT_STEP[args.precision]
+    bpp = stream_bytes_per_point(ks, desc0) or EXACT_BYTES_PER_POINT_STEP[args.precision]
     # the dominant kernel: the streaming stage kernel (the exact-order kernel
     # when the precision has no streaming form)
     if ks["stream_launches"] > 0 and ks["stream_ms"] > 0:
@@ -826,13 +834,13 @@ def main():
         kbytes = npts * bpp / 4.0 * ks["stages"]
     achieved = kbytes / (kms / 1e3) / 1e9 if kms > 0 else None
     # PML auxiliaries: every slab point below the free surface reads and
-    # writes 27 / 45 / 45 / 27 floats in stages 0..3 (144 B per stage on average)
+    # writes 18 / 27 / 45 / 27 floats in stages 0..3 (117 B per stage on average)
     npml = desc0.npml
     slab_pts = 0
     if npml > 0:
         kz = desc0.nz - 3
         slab_pts = 2 * npml * desc0.ny * kz + 2 * desc0.nx * npml * kz + desc0.nx * desc0.ny * npml
-    aux_bytes = slab_pts * 144.0 * klaunch if kname != "stage_exact_kernel" else 0.0
+    aux_bytes = slab_pts * 117.0 * klaunch if kname != "stage_exact_kernel" else 0.0
     achieved_pml = (kbytes + aux_bytes) / (kms / 1e3) / 1e9 if kms > 0 else None
     traffic = measured_traffic(w["name"], kname, args.precision, kbytes, klaunch)
 

@@ -199,8 +199,8 @@ int cgfdm_set_chunk(cgfdm_handle *h, int32_t planes);
 /* The fast path's configuration in use (after the autotuner, if it ran),
  * three values: form_chunk[0] = the streaming kernel's tile form 16, 8 or
  * 64; form_chunk[1] = planes per work item (0: automatic); form_chunk[2] = 1
- * if the free-surface layers run on the tiled kernel (the exact-order kernel
- * on the PML-slab columns), 0 if on the exact-order kernel alone.  All 0 when
+ * if the free-surface layers run on the tiled surface kernel, 0 if on the
+ * exact-order kernel (a tuning file can ask for that).  All 0 when
  * the handle runs the exact-order kernel only. */
 int cgfdm_get_tuning(cgfdm_handle *h, int32_t *form_chunk);
 
@@ -317,7 +317,7 @@ int cgfdm_server_destroy(cgfdm_server *s);
  * while they run -- a serving process that splits all of HBM into fixed pools
  * at start-up, or a framework whose allocator owns every byte of device
  * memory -- this runs the same stage as cgfdm_stage on a handle (streaming
- * kernel below the three free-surface layers, exact-order kernel for them)
+ * kernel below the three free-surface layers, surface kernel for them)
  * on buffers the caller already owns, and allocates nothing.  Its only
  * scratch (error flag, work-queue counter, PML profile table) is a fixed
  * 64 KiB device array per device, held by every GPU that loads the library.
