@@ -789,8 +789,7 @@ def main():
             pk16 = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))).get("hbm_gbs") \
                 if os.path.exists(os.path.join(ROOT, "MEASURED_PEAKS.json")) else None
             pk16 = pk16 or 6650.0
-            kn16 = {64: "stage_pair_kernel", 16: "stage_stream_batch_kernel",
-                    8: "stage_stream_kernel"}.get(form16, "stage_stream_kernel")
+            kn16 = "stage_pair_kernel" if form16 == 64 else "stage_stream_kernel"
             fp16["roofline"] = {"bound": "hbm", "achieved": a16, "peak": pk16, "unit": "GB/s",
                                 "frac": a16 / pk16,
                                 "traffic": measured_traffic(w["name"], kn16, "fp16",
@@ -824,9 +823,7 @@ def main():
     # the dominant kernel: the streaming stage kernel (the exact-order kernel
     # when the precision has no streaming form)
     if ks["stream_launches"] > 0 and ks["stream_ms"] > 0:
-        # tile height 16 runs the batched form of the kernel (a batch of one)
-        kname = {16: "stage_stream_batch_kernel", 8: "stage_stream_kernel",
-                 64: "stage_pair_kernel"}.get(form, "stage_stream_kernel")
+        kname = "stage_pair_kernel" if form == 64 else "stage_stream_kernel"
         kms, klaunch = ks["stream_ms"], ks["stream_launches"]
         kbytes = ks["stream_bytes"]
     else:
