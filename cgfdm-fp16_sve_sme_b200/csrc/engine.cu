@@ -29,6 +29,7 @@
 #include <string>
 #include <tuple>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "engine.h"
@@ -1342,12 +1343,13 @@ template <typename S> class BatchT : public BatchBase {
       tuned_ = true;
     }
     // a member whose model, sources, stations or form changed makes the
-    // captured steps stale
-    std::vector<unsigned> revs;
-    for (auto *m : m_) revs.push_back(m->rev_);
-    if (revs != revs_) {
+    // captured steps stale, and so does one that has advanced by itself: its
+    // signs are another step's then
+    std::vector<std::pair<unsigned, int>> held;
+    for (auto *m : m_) held.emplace_back(m->rev_, (int)(((m->it_ - count_) % 8 + 8) % 8));
+    if (held != held_) {
       drop_graphs();
-      revs_ = revs;
+      held_ = held;
     }
     for (int s = 0; s < nsteps; ++s) {
       const int p = count_ % 8;
@@ -1483,7 +1485,9 @@ template <typename S> class BatchT : public BatchBase {
   cudaGraphExec_t gexec_[8] = {};
   bool gseen_[8] = {};
   long long count_ = 0;  // steps run by this batch
-  std::vector<unsigned> revs_;  // members' rev_ when the graphs were captured
+  // what the captured steps hold of each member: its rev_ and its step minus
+  // the batch's, mod 8
+  std::vector<std::pair<unsigned, int>> held_;
   bool tuned_ = false;   // members' work-item depths chosen (first run)
 };
 
