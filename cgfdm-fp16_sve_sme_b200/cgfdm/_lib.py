@@ -116,6 +116,7 @@ SIGNATURES = {
     "cgfdm_setup_from_directory_ex": (C.c_int, [C.c_char_p, I32, C.POINTER(Setup)]),
     "cgfdm_free_setup": (C.c_int, [C.POINTER(Setup)]),
     "cgfdm_stage_noalloc": (C.c_int, [C.POINTER(StageBuffers), P, I32]),
+    "cgfdm_stage_noalloc_inject_fault": (C.c_int, [I32, P]),
 }
 
 

@@ -16,8 +16,9 @@
 //   [0, 4)     error flag.  Zero when the module loads; a kernel sets it when a
 //              bounded wait expires; only a call with wait != 0 reads it back
 //              and clears it.
-//   [4, 20)    the streaming kernels' two work queues.  Zero when the module
-//              loads, and every launch leaves its own at zero.
+//   [4, 20)    the streaming kernels' two work queues.  Every launch leaves its
+//              own at zero, and every call zeroes them before its launches:
+//              calls that overlap can leave them otherwise.
 //   [256, ...) PML profiles alpha, beta, d for x, y, z (3 x (_nx_+_ny_+_nz_)
 //              floats), rewritten by every call before its launches.  The
 //              values travel in the parameters of small fill kernels on the
@@ -48,6 +49,7 @@ namespace cgfdm {
 namespace {
 
 constexpr int kScratchBytes = 64 * 1024;
+constexpr int kQueueOffset = 4;
 constexpr int kProfileOffset = 256;
 constexpr int kMaxDevices = 64;
 
@@ -71,23 +73,27 @@ cudaError_t scratch_of(int dev, unsigned char **out) {
 }
 
 // Fill kernel for the profile table: its values arrive in the kernel's
-// parameter space (at most 32 KB), copied by the launch itself.
+// parameter space (at most 32 KB), copied by the launch itself.  The first
+// chunk's launch zeroes the work queues as well (queues: null in the others).
 constexpr int kFillChunk = 7936;
 struct FillChunk {
   int n;
   float v[kFillChunk];
 };
-__global__ void fill_profile_kernel(float *dst, const __grid_constant__ FillChunk c) {
+constexpr int kQueueInts = 4;
+__global__ void fill_profile_kernel(float *dst, int *queues, const __grid_constant__ FillChunk c) {
+  if (queues && blockIdx.x == 0 && threadIdx.x < kQueueInts) queues[threadIdx.x] = 0;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < c.n; q += gridDim.x * blockDim.x)
     dst[q] = c.v[q];
 }
 
-cudaError_t upload_profiles(float *dst, const std::vector<float> &prof, cudaStream_t st) {
+cudaError_t upload_profiles(float *dst, int *queues, const std::vector<float> &prof,
+                            cudaStream_t st) {
   static thread_local FillChunk c;
   for (size_t q0 = 0; q0 < prof.size(); q0 += kFillChunk) {
     c.n = (int)std::min<size_t>(kFillChunk, prof.size() - q0);
     std::memcpy(c.v, prof.data() + q0, sizeof(float) * c.n);
-    fill_profile_kernel<<<(c.n + 255) / 256, 256, 0, st>>>(dst + q0, c);
+    fill_profile_kernel<<<(c.n + 255) / 256, 256, 0, st>>>(dst + q0, q0 ? nullptr : queues, c);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -145,9 +151,9 @@ int stage_noalloc(const cgfdm_stage_buffers &b, cudaStream_t st, unsigned char *
     big = std::max(big, 9LL * n[0] * n[1] * n[2]);
   }
   // the profile table is rewritten by every call, through kernel parameters
-  NA_TRY(upload_profiles((float *)(scratch + kProfileOffset),
+  int *err = (int *)scratch, *counter = (int *)(scratch + kQueueOffset);
+  NA_TRY(upload_profiles((float *)(scratch + kProfileOffset), counter,
                          pml_profiles(b.nx, b.ny, b.nz, b.npml, b.dh), st));
-  int *err = (int *)scratch, *counter = (int *)(scratch + 4);
   // as a handle does: the exact-order kernel alone when opposite PML slabs
   // overlap (nPML above half the grid) or a slab is too large for the
   // streaming kernel's 32-bit auxiliary offsets
@@ -231,5 +237,19 @@ extern "C" int cgfdm_stage_noalloc(const cgfdm_stage_buffers *b, void *stream, i
     NA_TRY(cudaMemset(scratch, 0, sizeof flag));
     return fail(CGFDM_ERR_TIMEOUT, "a bounded device-side wait of the streaming kernel expired");
   }
+  return CGFDM_OK;
+}
+
+extern "C" int cgfdm_stage_noalloc_inject_fault(int32_t kind, void *stream) {
+  using namespace cgfdm;
+  if (kind != CGFDM_FAULT_STALE_QUEUES) return fail(CGFDM_ERR_ARG, "unknown fault kind");
+  int dev = 0;
+  NA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= kMaxDevices) return fail(CGFDM_ERR_ARG, "device index out of range");
+  unsigned char *scratch = nullptr;
+  NA_TRY(scratch_of(dev, &scratch));
+  // 0x01010101 in each int: no item left and a count that no launch resets
+  NA_TRY(cudaMemsetAsync(scratch + kQueueOffset, 1, kQueueInts * sizeof(int),
+                         (cudaStream_t)stream));
   return CGFDM_OK;
 }

@@ -341,18 +341,19 @@ int cgfdm_server_destroy(cgfdm_server *s);
  *
  * Limits and rules: precision FP32, FP16 or BF16; the PML profile table must
  * fit the scratch (nx + ny + nz + 18 <= 5440, else CGFDM_ERR_ARG).  All calls
- * on one device share the scratch and see what the last call left there
- * (every launch leaves its work queue empty), so calls whose work overlaps
- * on the GPU race.  The error flag starts at zero, is set by an
- * expired bounded wait, and is read and cleared only when `wait` is
- * non-zero: then the call synchronizes `stream` and returns CGFDM_ERR_TIMEOUT
- * if it was set.  With wait = 0 the call only enqueues work on `stream`
- * (current device): the profile table reaches the scratch through the
- * parameters of small fill kernels, not through a host-to-device copy.  The
- * first call on a device resolves the scratch address; make it before any
- * stream capture.  Each streaming-kernel variant has its shared-memory
- * attribute set on its first launch in the process.  A pointer that is not
- * 256-byte aligned is rejected with CGFDM_ERR_ARG.
+ * on one device share the scratch, so calls whose work overlaps on the GPU
+ * race.  Each call rewrites the profile table and empties the work queues
+ * before its launches: a call that overlaps no other is right whatever ran
+ * before it.  The error flag starts at zero, is set by an expired bounded
+ * wait, and is read and cleared only when `wait` is non-zero: then the call
+ * synchronizes `stream` and returns CGFDM_ERR_TIMEOUT if it was set.  With
+ * wait = 0 the call only enqueues work on `stream` (current device): the
+ * profile table reaches the scratch through the parameters of small fill
+ * kernels, not through a host-to-device copy.  The first call on a device
+ * resolves the scratch address; make it before any stream capture.  Each
+ * streaming-kernel variant has its shared-memory attribute set on its first
+ * launch in the process.  A pointer that is not 256-byte aligned is rejected
+ * with CGFDM_ERR_ARG.
  */
 typedef struct {
   int32_t nx, ny, nz, npml;
@@ -372,6 +373,13 @@ typedef struct {
 } cgfdm_stage_buffers;
 
 int cgfdm_stage_noalloc(const cgfdm_stage_buffers *b, void *stream, int32_t wait);
+
+/* Failure testing: leaves the scratch of the current device as overlapping
+ * calls can leave it, with work queues that are not empty (enqueued on
+ * `stream`).  The next cgfdm_stage_noalloc must be right all the same.  Any
+ * kind but CGFDM_FAULT_STALE_QUEUES is refused. */
+#define CGFDM_FAULT_STALE_QUEUES 2
+int cgfdm_stage_noalloc_inject_fault(int32_t kind, void *stream);
 
 /* Drop-in for propagate() with host buffers: uploads the model and sources,
  * runs all nt steps, returns station seismograms, the PGV map and the final
