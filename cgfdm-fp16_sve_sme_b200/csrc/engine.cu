@@ -16,6 +16,7 @@
 // planes below the three free-surface layers and the surface kernel those
 // (KERNEL_STREAM / AUTO); KERNEL_EXACT runs the exact-order
 // kernel everywhere (bit-identical to the reference's FP32 CPU build).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <unistd.h>
@@ -33,6 +34,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "fork.h"
 #include "json.h"
 #include "kernels.h"
 
@@ -52,6 +54,21 @@ const char *last_error() { return g_err.c_str(); }
       return e_ == cudaErrorMemoryAllocation ? CGFDM_ERR_NOMEM : CGFDM_ERR_CUDA;        \
     }                                                                                   \
   } while (0)
+
+bool stream_is_partitioned(cudaStream_t st) {
+  typedef CUresult (*Fn)(CUstream, CUgreenCtx *);
+  static const Fn fn = []() -> Fn {  // null on drivers without green contexts
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuStreamGetGreenCtx", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      return (Fn)p;
+    cudaGetLastError();
+    return nullptr;
+  }();
+  CUgreenCtx g = nullptr;
+  return fn && fn((CUstream)st, &g) == CUDA_SUCCESS && g != nullptr;
+}
 
 namespace {
 
@@ -179,83 +196,6 @@ Dims make_dims(const cgfdm_desc &d) {
 
 template <typename S> class BatchT;
 
-// Two side streams that branch off a caller's stream and join it again, for
-// the launches of one stage (its owner's host thread drives them).  Under
-// stream capture they become parallel branches of the graph.  An owner that
-// goes away leaves its idle streams and events to the next one (at most
-// kForkIdle sets are kept): creating them took 0.3 to 1.5 ms of a handle's 2.4.
-struct ForkSet {
-  int device = -1;
-  cudaStream_t side[2] = {};
-  cudaEvent_t start = nullptr, done[2] = {};
-  void destroy() {
-    for (int q = 0; q < 2; ++q) {
-      if (side[q]) cudaStreamDestroy(side[q]);
-      if (done[q]) cudaEventDestroy(done[q]);
-    }
-    if (start) cudaEventDestroy(start);
-  }
-};
-constexpr size_t kForkIdle = 32;
-std::mutex g_fork_mu;
-std::vector<ForkSet> g_fork_idle;
-
-class Fork {
- public:
-  cudaError_t create(int device) {
-    {
-      std::lock_guard<std::mutex> lk(g_fork_mu);
-      for (size_t q = 0; q < g_fork_idle.size(); ++q)
-        if (g_fork_idle[q].device == device) {
-          s_ = g_fork_idle[q];
-          g_fork_idle.erase(g_fork_idle.begin() + q);
-          return cudaSuccess;
-        }
-    }
-    s_.device = device;
-    cudaError_t e = cudaEventCreateWithFlags(&s_.start, cudaEventDisableTiming);
-    for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
-      e = cudaStreamCreateWithFlags(&s_.side[q], cudaStreamNonBlocking);
-      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s_.done[q], cudaEventDisableTiming);
-    }
-    return e;
-  }
-  void destroy() {  // the owner's device is current
-    if (s_.device < 0) return;
-    bool idle = s_.start && s_.done[0] && s_.done[1];
-    for (int q = 0; q < 2; ++q)
-      idle = s_.side[q] && cudaStreamSynchronize(s_.side[q]) == cudaSuccess && idle;
-    if (idle) {
-      std::lock_guard<std::mutex> lk(g_fork_mu);
-      if (g_fork_idle.size() < kForkIdle) {
-        g_fork_idle.push_back(s_);
-        s_ = ForkSet();
-        return;
-      }
-    }
-    s_.destroy();
-    s_ = ForkSet();
-  }
-  cudaError_t begin(cudaStream_t st) {
-    cudaError_t e = cudaEventRecord(s_.start, st);
-    for (int q = 0; q < 2 && e == cudaSuccess; ++q) e = cudaStreamWaitEvent(s_.side[q], s_.start, 0);
-    return e;
-  }
-  cudaError_t end(cudaStream_t st) {
-    cudaError_t e = cudaSuccess;
-    for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
-      e = cudaEventRecord(s_.done[q], s_.side[q]);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, s_.done[q], 0);
-    }
-    return e;
-  }
-  cudaStream_t side(int q) const { return s_.side[q]; }
-  StreamPair pair(cudaStream_t st) const { return {st, s_.side[1]}; }
-
- private:
-  ForkSet s_;
-};
-
 template <typename S> class EngineT : public Engine {
   using R = typename Arith<S>::R;
   friend class BatchT<S>;
@@ -296,7 +236,6 @@ template <typename S> class EngineT : public Engine {
     // queues, [5] set_model's check
     CUDA_TRY(cudaMalloc(&err_flag_, 6 * sizeof(int)));
     CUDA_TRY(cudaMemsetAsync(err_flag_, 0, 6 * sizeof(int), own_stream_));
-    CUDA_TRY(fork_.create(d_.device));
     // the device copy of the step counter it_ (read by the per-step kernels)
     CUDA_TRY(cudaMalloc(&step_, 2 * sizeof(int)));  // the step, the end-of-step block counter
     CUDA_TRY(cudaMemsetAsync(step_, 0, 2 * sizeof(int), own_stream_));
@@ -315,6 +254,7 @@ template <typename S> class EngineT : public Engine {
       return CGFDM_ERR_ARG;
     }
     if (use_stream_) {
+      CUDA_TRY(fork_.attach(own_stream_));
       S *bufs[3] = {A_, X_, Y_};
       for (int b = 0; b < 3; ++b) {
         int rc = encode_stream_maps<S>(bufs[b], cjm_, A_, T_, X_, g_.L, tmap_[b]);
@@ -474,6 +414,7 @@ template <typename S> class EngineT : public Engine {
     // work queued earlier on another stream (a batch, another caller) first
     if (last_stream_ && last_stream_ != st) CUDA_TRY(cudaStreamSynchronize(last_stream_));
     last_stream_ = st;
+    if (use_stream_) CUDA_TRY(fork_.attach(st));
     if (use_stream_ && tile_rows_ == 0) {
       int rc = tune(st);
       if (rc) return rc;
@@ -578,6 +519,7 @@ template <typename S> class EngineT : public Engine {
     int fb[3] = {fb1, fb2, fb3};
     if (last_stream_ && last_stream_ != st) CUDA_TRY(cudaStreamSynchronize(last_stream_));
     last_stream_ = st;
+    if (use_stream_) CUDA_TRY(fork_.attach(st));
     return launch_stage(irk, fb, st, false);
   }
 
@@ -1015,11 +957,12 @@ template <typename S> class EngineT : public Engine {
         b0.chunk = b1.chunk = ch;
         auto pair = [&]() {
           for (int q = 0; q < 2; ++q) {
-            cudaError_t e = fork_.begin(st);
+            Branches br(fork_, st, false);
+            cudaError_t e = br.begin();
             if (e == cudaSuccess)
               e = launch_stage_stream<S>(q ? b1 : b0, tmap_[q], err_flag_, err_flag_ + 1,
-                                         fork_.pair(st), nullptr, nullptr, rows);
-            if (e == cudaSuccess) e = fork_.end(st);
+                                         StreamPair{st, br.side(1)}, nullptr, nullptr, rows);
+            if (e == cudaSuccess) e = br.join();
             if (e != cudaSuccess) return e;
           }
           return cudaSuccess;
@@ -1077,19 +1020,18 @@ template <typename S> class EngineT : public Engine {
       // and read none of each other's: the first two run on side streams, so
       // that they fill the SMs which the others leave idle (timed runs keep
       // them in turn, to time each).
-      if (!ev) CUDA_TRY(fork_.begin(st));
-      const cudaStream_t side = ev ? st : fork_.side(0);
+      Branches br(fork_, st, ev != nullptr);
+      CUDA_TRY(br.begin());
+      const cudaStream_t side = br.side(0);
       if (!ev) CUDA_TRY(fast_top_ ? launch_surface(&a, 1, side) : launch_surface_exact(a, side));
       CUDA_TRY(launch_stage_stream<S>(b, tmap_[in_of[irk]], err_flag_, err_flag_ + 1,
-                                      ev ? StreamPair{st, st} : fork_.pair(st),
-                                      ev ? ev[1] : nullptr, &launches_,
-                                      tile_rows_ ? tile_rows_ : 16));
+                                      StreamPair{st, br.side(1)}, ev ? ev[1] : nullptr,
+                                      &launches_, tile_rows_ ? tile_rows_ : 16));
       if (ev) {
         CUDA_TRY(cudaEventRecord(ev[2], st));
         CUDA_TRY(fast_top_ ? launch_surface(&a, 1, side) : launch_surface_exact(a, side));
-      } else {
-        CUDA_TRY(fork_.end(st));
       }
+      CUDA_TRY(br.join());
       // fields read and written per point by this stage: W in, 12 coefficients
       // (8 on a vertically stretched grid), W out, plus m (stages 1, 2), stage
       // 1's input (2) and t (written in 2, read in 3)
@@ -1307,7 +1249,6 @@ template <typename S> class BatchT : public BatchBase {
     CUDA_TRY(cudaStreamCreateWithFlags(&own_, cudaStreamNonBlocking));
     CUDA_TRY(cudaMalloc(&err_, 5 * sizeof(int)));
     CUDA_TRY(cudaMemsetAsync(err_, 0, 5 * sizeof(int), own_));
-    CUDA_TRY(fork_.create(dev_));
     CUDA_TRY(cudaStreamSynchronize(own_));
     return CGFDM_OK;
   }
@@ -1327,6 +1268,7 @@ template <typename S> class BatchT : public BatchBase {
         return CGFDM_ERR_ARG;
       }
     last_ = st;
+    CUDA_TRY(fork_.attach(st));
     for (auto *m : m_) {
       // members' own work (uploads, earlier runs) comes first on this stream
       if (m->last_stream_ && m->last_stream_ != st) CUDA_TRY(cudaStreamSynchronize(m->last_stream_));
@@ -1337,6 +1279,7 @@ template <typename S> class BatchT : public BatchBase {
       // every member's work-item depth for the batch's 32 x 8 form
       for (auto *m : m_)
         if (m->use_stream_ && !m->chunk_fixed_) {
+          CUDA_TRY(m->fork_.attach(st));
           int rc = m->tune(st, true);
           if (rc) return rc;
         }
@@ -1395,7 +1338,8 @@ template <typename S> class BatchT : public BatchBase {
     std::vector<StageArgs<S>> args;
     std::vector<const void *> maps;
     for (int irk = 0; irk < 4; ++irk) {
-      CUDA_TRY(fork_.begin(st));
+      Branches br(fork_, st, false);
+      CUDA_TRY(br.begin());
       // the free-surface layers (and members on the exact-order kernel) beside
       // the streaming launches, as in launch_stage
       args.clear();
@@ -1407,14 +1351,14 @@ template <typename S> class BatchT : public BatchBase {
           if (m->fast_top_)
             args.push_back(a);
           else
-            CUDA_TRY(m->launch_surface_exact(a, fork_.side(0)));
+            CUDA_TRY(m->launch_surface_exact(a, br.side(0)));
         } else {
-          int rc = m->launch_stage(irk, fb, fork_.side(0), true);
+          int rc = m->launch_stage(irk, fb, br.side(0), true);
           if (rc) return rc;
         }
       }
       if (!args.empty())
-        CUDA_TRY(m_[0]->launch_surface(args.data(), (int)args.size(), fork_.side(0)));
+        CUDA_TRY(m_[0]->launch_surface(args.data(), (int)args.size(), br.side(0)));
       for (int code = 0; code < 16; ++code) {
         args.clear();
         maps.clear();
@@ -1432,9 +1376,9 @@ template <typename S> class BatchT : public BatchBase {
         }
         if (!args.empty())
           CUDA_TRY(launch_stage_stream_batch<S>(args.data(), maps.data(), (int)args.size(), err_,
-                                                err_ + 1, fork_.pair(st)));
+                                                err_ + 1, StreamPair{st, br.side(1)}));
       }
-      CUDA_TRY(fork_.end(st));
+      CUDA_TRY(br.join());
     }
     for (auto *m : m_) {
       int rc = m->step_end(st);

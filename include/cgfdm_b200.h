@@ -120,7 +120,12 @@ int cgfdm_set_stations(cgfdm_handle *h, const int32_t *xyz, int32_t nsta);
 
 /* Advances nsteps time steps (sources, 4 RK stages, stations, PGV) on the
  * CUDA stream `stream` (a cudaStream_t, NULL = the handle's own stream).
- * Asynchronous: returns once the work is enqueued. */
+ * Asynchronous: returns once the work is enqueued.  Launches of a stage that
+ * do not depend on each other branch off `stream` onto side streams of the
+ * same priority, which join it again before the next stage, also when the
+ * call fails.  On a stream of an SM partition (a green context) every launch
+ * goes to `stream` itself, one after the other.  The same holds for
+ * cgfdm_stage and cgfdm_batch_run. */
 int cgfdm_run(cgfdm_handle *h, int32_t nsteps, void *stream);
 
 /* One RK stage irk (0..3) with MacCormack signs fb1..fb3 and no source,
