@@ -21,6 +21,7 @@
 
 #include <unistd.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -907,12 +908,18 @@ template <typename S> class EngineT : public Engine {
   // Picks the streaming kernel's tile form (32 x 16, 32 x 8, and for 16-bit
   // storage the paired-point 64 x 8 form) and work-item depth in z (automatic,
   // 64 or 32 planes; the depth set by cgfdm_set_chunk is kept) for this grid
-  // and precision: times the streaming part of stages 0 and 1 at the current
-  // step boundary with each candidate and keeps the fastest.  Stage 0 reads
-  // only the step state A and step-start auxiliaries and writes X, T and the
-  // stage-1 auxiliary inputs; stage 1 reads those and writes Y and T; the
-  // real step rewrites all of them before reading them, so the timing leaves
-  // the run unchanged (as stages of a whole step they leave T alone).  Results are cached per (precision, grid).
+  // and precision: times the streaming part of stages 0, 1 and 2 of a whole
+  // step at the current step boundary with each candidate and keeps the one
+  // with the least mean (a candidate whose time varies costs its mean).  Each
+  // of the three stages is a kernel of its own (see stage_of in
+  // stage_stream.cuh) and stage 2 moves the most: at 1201x1201x401 in FP16
+  // items of 64 planes take 14.5 ms there against 16.2 to 17.3 for the automatic
+  // depth, which is 1 to 2 % ahead in stages 0 and 1.  They read the
+  // step state A, the step-start auxiliaries and each other's results, and
+  // write X, Y, T and the auxiliaries of those; the real step rewrites all of
+  // them before reading them, so the timing leaves the run unchanged.
+  // Stage 3, which ends the step in A, is not timed.  Results are cached per
+  // (precision, grid).
   // batch_form: a batch member, which always runs the 32 x 8 form inside
   // its batch; only the depth is chosen and the member's own form is kept.
   int tune(cudaStream_t st, bool batch_form = false) {
@@ -936,8 +943,6 @@ template <typename S> class EngineT : public Engine {
         return CGFDM_OK;
       }
     }
-    const int fb0[3] = {kFB[it_ % 8][0], kFB[it_ % 8][1], kFB[it_ % 8][2]};
-    const int fb1[3] = {-fb0[0], -fb0[1], -fb0[2]};
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     CUDA_TRY(cudaEventCreate(&e0));
     CUDA_TRY(cudaEventCreate(&e1));
@@ -946,48 +951,60 @@ template <typename S> class EngineT : public Engine {
     if (batch_form) forms = {8};
     std::vector<int> chunks = {0, 64, 32};
     if (chunk_fixed_) chunks = {chunk_};
-    int best_form = 16, best_chunk = chunks[0];
-    float best_ms = 1e30f;
-    cudaError_t err = cudaSuccess;
+    struct Candidate {
+      int form, chunk;
+      float ms;  // all its timed rounds
+    };
+    std::vector<Candidate> cand;
     for (int rows : forms)
-      for (int ch : chunks) {
-        StageArgs<S> b0 = stage_args(0, fb0, true), b1 = stage_args(1, fb1, true);
-        b0.kbeg = b1.kbeg = HALO;
-        b0.kend = b1.kend = g_.L.nz_ - HALO - 3;
-        b0.chunk = b1.chunk = ch;
-        auto pair = [&]() {
-          for (int q = 0; q < 2; ++q) {
-            Branches br(fork_, st, false);
-            cudaError_t e = br.begin();
-            if (e == cudaSuccess)
-              e = launch_stage_stream<S>(q ? b1 : b0, tmap_[q], err_flag_, err_flag_ + 1,
-                                         StreamPair{st, br.side(1)}, nullptr, nullptr, rows);
-            if (e == cudaSuccess) e = br.join();
-            if (e != cudaSuccess) return e;
-          }
-          return cudaSuccess;
-        };
-        err = pair();
+      for (int ch : chunks) cand.push_back({rows, ch, 0.0f});
+    auto stages = [&](const Candidate &c) {
+      for (int irk = 0; irk < 3; ++irk) {
+        int fb[3];
+        step_fb(irk, fb);
+        StageArgs<S> b = stage_args(irk, fb, true);
+        b.kbeg = HALO;
+        b.kend = g_.L.nz_ - HALO - 3;
+        b.chunk = c.chunk;
+        Branches br(fork_, st, false);
+        cudaError_t e = br.begin();
+        if (e == cudaSuccess)  // the input of stage irk is buffer irk
+          e = launch_stage_stream<S>(b, tmap_[irk], err_flag_, err_flag_ + 1,
+                                     StreamPair{st, br.side(1)}, nullptr, nullptr, c.form);
+        if (e == cudaSuccess) e = br.join();
+        if (e != cudaSuccess) return e;
+      }
+      return cudaSuccess;
+    };
+    // rounds over the candidates, the first of them untimed: at least three
+    // timed ones, and up to eight until a candidate's take 2 ms together.  A
+    // candidate that the first timed round has a tenth behind drops out.
+    cudaError_t err = cudaSuccess;
+    for (int round = 0; err == cudaSuccess; ++round) {
+      for (Candidate &c : cand) {
+        float one = 0;
         if (err == cudaSuccess) err = cudaEventRecord(e0, st);
-        for (int r = 0; r < 2 && err == cudaSuccess; ++r) err = pair();
+        if (err == cudaSuccess) err = stages(c);
         if (err == cudaSuccess) err = cudaEventRecord(e1, st);
         if (err == cudaSuccess) err = cudaEventSynchronize(e1);
-        float ms = 0;
-        if (err == cudaSuccess) err = cudaEventElapsedTime(&ms, e0, e1);
-        if (err != cudaSuccess) break;
-        if (ms < best_ms) {
-          best_ms = ms;
-          best_form = rows;
-          best_chunk = ch;
-        }
+        if (err == cudaSuccess) err = cudaEventElapsedTime(&one, e0, e1);
+        if (round > 0) c.ms += one;
       }
+      if (round == 0 || err != cudaSuccess) continue;
+      std::stable_sort(cand.begin(), cand.end(),
+                       [](const Candidate &x, const Candidate &y) { return x.ms < y.ms; });
+      if (round == 1)
+        while (cand.back().ms > 1.1f * cand.front().ms) cand.pop_back();
+      if (cand.size() == 1 || (round >= 3 && cand.front().ms >= 2.0f) || round == 8) break;
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     CUDA_TRY(err);
-    if (!batch_form) tile_rows_ = best_form;
-    chunk_ = best_chunk;
+    const Candidate best = cand.front();
+    if (!batch_form) tile_rows_ = best.form;
+    chunk_ = best.chunk;
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tuned[key] = {best_form, best_chunk, fast_top_};
+    g_tuned[key] = {best.form, best.chunk, fast_top_};
     if (!cache.empty()) tune_cache_store(cache, tune_cache_key(d_.device, key), g_tuned[key]);
     return CGFDM_OK;
   }
