@@ -76,23 +76,31 @@ namespace {
 const int kFB[8][3] = {{-1, -1, -1}, {1, 1, -1}, {1, 1, 1},  {-1, -1, 1},
                        {-1, 1, -1},  {1, -1, -1}, {1, -1, 1}, {-1, 1, 1}};
 
-// Autotuner results: streaming-kernel tile height per (precision, nx, ny, nz,
-// nPML), shared by every handle of the process.
+// Autotuner results, shared by every handle of the process: the tile form and
+// work-item depth per (device, precision, nx, ny, nz, nPML, fixed depth or -1,
+// batch member, grid stretched in z only), what the timed kernels depend on.
 std::mutex g_tune_mu;
-// autotuned (tile form, work-item depth) per (precision, nx, ny, nz, nPML,
-// fixed depth or -1, batch member)
 struct Tuned {
   int form, chunk;
   bool fast_top;  // free-surface layers on the tiled kernel (else the exact-order kernel)
 };
-std::map<std::tuple<int, int, int, int, int, int, int>, Tuned> g_tuned;
+struct TuneKey {
+  int device, precision, nx, ny, nz, npml, chunk, batch, vert;
+  auto all() const { return std::tie(device, precision, nx, ny, nz, npml, chunk, batch, vert); }
+  bool operator<(const TuneKey &o) const { return all() < o.all(); }
+};
+std::map<TuneKey, Tuned> g_tuned;
+// Part of the keys in a tuning file: raised when the kernels or what the tuner
+// times change, so that choices made for others are not taken.
+constexpr int kTuneRevision = 2;
 
 // Tuning choices kept across processes (optional).  When the environment
 // variable CGFDM_TUNE_CACHE names a file, a tuner that has no choice for its
 // key in this process looks it up there before timing anything, and every
 // choice it times is written back.  The file is a JSON object whose members
-// map a key naming the GPU (name and SM count), the precision, the grid, the
-// PML width, a fixed work-item depth (or -1) and batch membership to
+// map a key naming the GPU (name and SM count), kTuneRevision, the precision,
+// the grid, the PML width, a fixed work-item depth (or -1), batch membership
+// and the kind of grid (stretched in z only or general) to
 // [tile form, work-item depth, tiled free-surface kernel 0/1] (the tuner
 // writes 1 there; 0 in a file selects the exact-order kernel).  A malformed
 // file or entry is ignored (the tuner times as if it were absent); writers
@@ -103,13 +111,14 @@ std::string tune_cache_path() {
   const char *p = std::getenv("CGFDM_TUNE_CACHE");
   return p && *p ? std::string(p) : std::string();
 }
-std::string tune_cache_key(int device, const std::tuple<int, int, int, int, int, int, int> &k) {
+std::string tune_cache_key(const TuneKey &k) {
   cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return std::string();
+  if (cudaGetDeviceProperties(&prop, k.device) != cudaSuccess) return std::string();
   char buf[512];
-  std::snprintf(buf, sizeof buf, "%s|sm%d|precision%d|%dx%dx%d|npml%d|chunk%d|batch%d", prop.name,
-                prop.multiProcessorCount, std::get<0>(k), std::get<1>(k), std::get<2>(k),
-                std::get<3>(k), std::get<4>(k), std::get<5>(k), std::get<6>(k));
+  std::snprintf(buf, sizeof buf,
+                "%s|sm%d|rev%d|precision%d|%dx%dx%d|npml%d|chunk%d|batch%d|%s", prop.name,
+                prop.multiProcessorCount, kTuneRevision, k.precision, k.nx, k.ny, k.nz, k.npml,
+                k.chunk, k.batch, k.vert ? "vertical" : "general");
   for (char *c = buf; *c; ++c)
     if (*c == '"' || *c == '\\' || (unsigned char)*c < 0x20) *c = '_';
   return buf;
@@ -278,6 +287,13 @@ template <typename S> class EngineT : public Engine {
     CUDA_TRY(cudaMemcpyAsync(&lateral, err_flag_ + 5, sizeof(int), cudaMemcpyDeviceToHost,
                              own_stream_));
     CUDA_TRY(cudaStreamSynchronize(own_stream_));
+    if (vert_ != (lateral == 0) && form_tuned_) {
+      // other kernels from here on: the next run() chooses again
+      tile_rows_ = 0;
+      fast_top_ = true;
+      form_tuned_ = false;
+      if (!chunk_fixed_) chunk_ = 0;
+    }
     vert_ = lateral == 0;
     drop_graphs();
     std::vector<R> r(rdz, rdz + 18 * g_.nsurf);
@@ -768,6 +784,7 @@ template <typename S> class EngineT : public Engine {
       return CGFDM_ERR_ARG;
     }
     tile_rows_ = rows;
+    form_tuned_ = false;
     drop_graphs();
     return CGFDM_OK;
   }
@@ -918,26 +935,27 @@ template <typename S> class EngineT : public Engine {
   // step state A, the step-start auxiliaries and each other's results, and
   // write X, Y, T and the auxiliaries of those; the real step rewrites all of
   // them before reading them, so the timing leaves the run unchanged.
-  // Stage 3, which ends the step in A, is not timed.  Results are cached per
-  // (precision, grid).
+  // Stage 3, which ends the step in A, is not timed.  Results are cached, see
+  // TuneKey.
   // batch_form: a batch member, which always runs the 32 x 8 form inside
   // its batch; only the depth is chosen and the member's own form is kept.
   int tune(cudaStream_t st, bool batch_form = false) {
-    const auto key = std::make_tuple((int)d_.precision, d_.nx, d_.ny, d_.nz, d_.npml,
-                                     chunk_fixed_ ? chunk_ : -1, batch_form ? 1 : 0);
+    const TuneKey key{d_.device, (int)d_.precision, d_.nx, d_.ny, d_.nz, d_.npml,
+                      chunk_fixed_ ? chunk_ : -1, batch_form ? 1 : 0, vert_ ? 1 : 0};
     const std::string cache = tune_cache_path();
     {
       std::lock_guard<std::mutex> lk(g_tune_mu);
       auto f = g_tuned.find(key);
       if (f == g_tuned.end() && !cache.empty()) {
         Tuned t;
-        if (tune_cache_load(cache, tune_cache_key(d_.device, key), (int)sizeof(S), t))
+        if (tune_cache_load(cache, tune_cache_key(key), (int)sizeof(S), t))
           f = g_tuned.emplace(key, t).first;
       }
       if (f != g_tuned.end()) {
         if (!batch_form) {
           tile_rows_ = f->second.form;
           fast_top_ = f->second.fast_top;
+          form_tuned_ = true;
         }
         chunk_ = f->second.chunk;
         return CGFDM_OK;
@@ -1001,11 +1019,14 @@ template <typename S> class EngineT : public Engine {
     cudaEventDestroy(e1);
     CUDA_TRY(err);
     const Candidate best = cand.front();
-    if (!batch_form) tile_rows_ = best.form;
+    if (!batch_form) {
+      tile_rows_ = best.form;
+      form_tuned_ = true;
+    }
     chunk_ = best.chunk;
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tuned[key] = {best.form, best.chunk, fast_top_};
-    if (!cache.empty()) tune_cache_store(cache, tune_cache_key(d_.device, key), g_tuned[key]);
+    if (!cache.empty()) tune_cache_store(cache, tune_cache_key(key), g_tuned[key]);
     return CGFDM_OK;
   }
 
@@ -1212,6 +1233,7 @@ template <typename S> class EngineT : public Engine {
   bool vert_ = false;         // see StageArgs::vert; false until a model is set
   unsigned rev_ = 0;          // counts what makes captured steps stale
   bool fast_top_ = true;      // free-surface layers on the tiled kernel (see Tuned)
+  bool form_tuned_ = false;   // tile_rows_ is the autotuner's choice
   bool chunk_fixed_ = false;  // set by set_chunk: the autotuner keeps chunk_
   bool drop_next_load_ = false;  // fault injection for failure-detection tests
   int *step_ = nullptr;       // device copy of it_, then the end-of-step kernel's block counter
@@ -1292,15 +1314,18 @@ template <typename S> class BatchT : public BatchBase {
       CUDA_TRY(cudaStreamSynchronize(m->own_stream_));
       m->last_stream_ = st;
     }
-    if (!tuned_) {
-      // every member's work-item depth for the batch's 32 x 8 form
-      for (auto *m : m_)
-        if (m->use_stream_ && !m->chunk_fixed_) {
-          CUDA_TRY(m->fork_.attach(st));
-          int rc = m->tune(st, true);
-          if (rc) return rc;
-        }
-      tuned_ = true;
+    // every member's work-item depth for the batch's 32 x 8 form, again when a
+    // new model of the other kind was set
+    tuned_for_.resize(m_.size(), -1);
+    for (size_t q = 0; q < m_.size(); ++q) {
+      EngineT<S> *m = m_[q];
+      if (tuned_for_[q] == (int)m->vert_) continue;
+      if (m->use_stream_ && !m->chunk_fixed_) {
+        CUDA_TRY(m->fork_.attach(st));
+        int rc = m->tune(st, true);
+        if (rc) return rc;
+      }
+      tuned_for_[q] = m->vert_;
     }
     // a member whose model, sources, stations or form changed makes the
     // captured steps stale, and so does one that has advanced by itself: its
@@ -1449,7 +1474,7 @@ template <typename S> class BatchT : public BatchBase {
   // what the captured steps hold of each member: its rev_ and its step minus
   // the batch's, mod 8
   std::vector<std::pair<unsigned, int>> held_;
-  bool tuned_ = false;   // members' work-item depths chosen (first run)
+  std::vector<int> tuned_for_;  // members' vert_ when their depths were chosen (-1: not yet)
 };
 
 template <typename S>
