@@ -1255,7 +1255,8 @@ int64_t engine_device_bytes(const cgfdm_desc &d) {
   int64_t r = d.precision == CGFDM_FP64 ? 8 : 4;
   int64_t aux = 0;
   for (int q = 0; q < 5; ++q) aux += g.slab_pts[q] * 9;
-  return s * (4 * 9 + 13) * g.L.fs + r * (18 * g.nsurf + 4 * aux) + 8 * (int64_t)d.nx * d.ny;
+  // the PGV map and get_free_surface's staging: two and three floats a column
+  return s * (4 * 9 + 13) * g.L.fs + r * (18 * g.nsurf + 4 * aux) + 20 * (int64_t)d.nx * d.ny;
 }
 
 namespace {
