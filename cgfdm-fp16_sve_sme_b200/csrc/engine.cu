@@ -264,7 +264,7 @@ template <typename S> class EngineT : public Engine {
       return CGFDM_ERR_ARG;
     }
     if (use_stream_) {
-      CUDA_TRY(fork_.attach(own_stream_));
+      CUDA_TRY(fork_.attach(d_.device, own_stream_));
       S *bufs[3] = {A_, X_, Y_};
       for (int b = 0; b < 3; ++b) {
         int rc = encode_stream_maps<S>(bufs[b], cjm_, A_, T_, X_, g_.L, tmap_[b]);
@@ -431,7 +431,7 @@ template <typename S> class EngineT : public Engine {
     // work queued earlier on another stream (a batch, another caller) first
     if (last_stream_ && last_stream_ != st) CUDA_TRY(cudaStreamSynchronize(last_stream_));
     last_stream_ = st;
-    if (use_stream_) CUDA_TRY(fork_.attach(st));
+    if (use_stream_) CUDA_TRY(fork_.attach(d_.device, st));
     if (use_stream_ && tile_rows_ == 0) {
       int rc = tune(st);
       if (rc) return rc;
@@ -536,7 +536,7 @@ template <typename S> class EngineT : public Engine {
     int fb[3] = {fb1, fb2, fb3};
     if (last_stream_ && last_stream_ != st) CUDA_TRY(cudaStreamSynchronize(last_stream_));
     last_stream_ = st;
-    if (use_stream_) CUDA_TRY(fork_.attach(st));
+    if (use_stream_) CUDA_TRY(fork_.attach(d_.device, st));
     return launch_stage(irk, fb, st, false);
   }
 
@@ -1308,7 +1308,7 @@ template <typename S> class BatchT : public BatchBase {
         return CGFDM_ERR_ARG;
       }
     last_ = st;
-    CUDA_TRY(fork_.attach(st));
+    CUDA_TRY(fork_.attach(dev_, st));
     for (auto *m : m_) {
       // members' own work (uploads, earlier runs) comes first on this stream
       if (m->last_stream_ && m->last_stream_ != st) CUDA_TRY(cudaStreamSynchronize(m->last_stream_));
@@ -1322,7 +1322,7 @@ template <typename S> class BatchT : public BatchBase {
       EngineT<S> *m = m_[q];
       if (tuned_for_[q] == (int)m->vert_) continue;
       if (m->use_stream_ && !m->chunk_fixed_) {
-        CUDA_TRY(m->fork_.attach(st));
+        CUDA_TRY(m->fork_.attach(dev_, st));
         int rc = m->tune(st, true);
         if (rc) return rc;
       }

@@ -1,7 +1,8 @@
 """The side streams of a stage (csrc/fork.h), compiled here against a stand-in
 for the CUDA runtime that writes down each call: they have the priority of the
-caller's stream, a stream of an SM partition gets none, and a stage that ends
-early on an error still makes the caller's stream wait for their work."""
+caller's stream, a stream of an SM partition gets none, a stage that ends
+early on an error still makes the caller's stream wait for their work, and the
+pool of idle ones is bounded."""
 import os
 import shutil
 import subprocess
@@ -14,7 +15,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 RUNTIME = r"""
 #pragma once
 #include <cstdio>
-struct FakeStream { const char *name; int prio; bool part; };
+struct FakeStream { const char *name; int prio; bool part, broken; };
 struct FakeEvent { int id; };
 typedef FakeStream *cudaStream_t;
 typedef FakeEvent *cudaEvent_t;
@@ -26,10 +27,14 @@ inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
 }
 inline cudaError_t cudaEventDestroy(cudaEvent_t e) { delete e; --g_live; return cudaSuccess; }
 inline cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned, int p) {
-  static const char *names[] = {"s0", "s1", "s2", "s3", "s4", "s5"};
-  *s = new FakeStream{names[g_streams++], p, false}; ++g_live; return cudaSuccess;
+  static char names[400][8];
+  std::snprintf(names[g_streams], sizeof names[0], "s%d", g_streams);
+  *s = new FakeStream{names[g_streams++], p, false, false}; ++g_live; return cudaSuccess;
 }
 inline cudaError_t cudaStreamDestroy(cudaStream_t s) { delete s; --g_live; return cudaSuccess; }
+inline cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+  return s->broken ? cudaErrorUnknown : cudaSuccess;
+}
 inline cudaError_t cudaStreamGetPriority(cudaStream_t s, int *p) { *p = s->prio; return cudaSuccess; }
 inline cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
   std::printf("record %d on %s\n", e->id, s->name); return cudaSuccess;
@@ -53,11 +58,11 @@ static int stage(Fork &f, cudaStream_t st, bool fails, bool in_turn = false) {
   return br.join() == cudaSuccess ? 0 : 1;
 }
 int main() {
-  FakeStream a{"a", 0, false}, high{"high", -5, false}, part{"part", 0, true};
+  FakeStream a{"a", 0, false, false}, high{"high", -5, false, false}, part{"part", 0, true, false};
   Fork f;
   for (cudaStream_t st : {&a, &high, &part, &a}) {
     std::printf("# %s\n", st->name);
-    if (f.attach(st) != cudaSuccess) return 1;
+    if (f.attach(0, st) != cudaSuccess) return 1;
     if (f.set()) std::printf("priorities %d %d\n", f.set()->side[0]->prio, f.set()->side[1]->prio);
     stage(f, st, false);
   }
@@ -66,13 +71,24 @@ int main() {
   std::printf("# in turn\n");
   stage(f, &a, false, true);
   std::printf("# branch refused\n");
-  struct Guard { ~Guard() { g_fail_wait = -1; } } g;
-  FakeStream b{"b", 3, false};
-  f.attach(&b);
   g_fail_wait = f.set()->start->id;
-  std::printf("rc %d\n", stage(f, &b, false));
+  std::printf("rc %d\n", stage(f, &a, false));
+  g_fail_wait = -1;
   f.destroy();
-  std::printf("# live %d\n", g_live);
+  std::printf("# pooled %d\n", g_live);
+  Fork h, other;
+  h.attach(0, &high);
+  other.attach(1, &a);
+  std::printf("# next owner %s, another device %s\n", h.set()->side[0]->name,
+              other.set()->side[0]->name);
+  h.set()->side[1]->broken = true;
+  h.destroy();
+  other.destroy();
+  std::printf("# after an error %d\n", g_live);
+  static Fork many[40];
+  for (Fork &m : many) m.attach(0, &a);
+  for (Fork &m : many) m.destroy();
+  std::printf("# at most %d\n", g_live);
 }
 """
 
@@ -128,5 +144,9 @@ def test_a_failing_stage_joins_its_branches(said):
     assert said["branch refused"][0][-1] == "rc 1"
 
 
-def test_every_stream_and_event_is_destroyed(said):
-    assert "live 0" in said
+def test_idle_sets_go_to_the_next_owner_of_the_device(said):
+    """Five streams and events a set; at most 32 sets are kept, none that an
+    error left behind, and none for another device or priority."""
+    assert "pooled 10" in said and "next owner s2, another device s4" in said
+    assert "after an error 10" in said  # the broken set went, the other device's stays
+    assert "at most %d" % (32 * 5) in said
