@@ -927,8 +927,8 @@ template <typename S> class EngineT : public Engine {
   // 64 or 32 planes; the depth set by cgfdm_set_chunk is kept) for this grid
   // and precision: times the streaming part of stages 0, 1 and 2 of a whole
   // step at the current step boundary with each candidate and keeps the one
-  // with the least mean (a candidate whose time varies costs its mean).  Each
-  // of the three stages is a kernel of its own (see stage_of in
+  // with the least mean (the least time falls for a candidate whose time
+  // varies).  Each of the three stages is a kernel of its own (see stage_of in
   // stage_stream.cuh) and stage 2 moves the most: at 1201x1201x401 in FP16
   // items of 64 planes take 14.5 ms there against 16.2 to 17.3 for the automatic
   // depth, which is 1 to 2 % ahead in stages 0 and 1.  They read the
@@ -971,7 +971,13 @@ template <typename S> class EngineT : public Engine {
     if (chunk_fixed_) chunks = {chunk_};
     struct Candidate {
       int form, chunk;
-      float ms;  // all its timed rounds
+      std::vector<float> ms;  // its timed rounds
+      float least() const { return *std::min_element(ms.begin(), ms.end()); }
+      float mean() const {  // a stall of the host counts as a quarter at most
+        float sum = 0, most = 1.25f * least();
+        for (float v : ms) sum += std::min(v, most);
+        return sum / ms.size();
+      }
     };
     std::vector<Candidate> cand;
     for (int rows : forms)
@@ -995,8 +1001,8 @@ template <typename S> class EngineT : public Engine {
       return cudaSuccess;
     };
     // rounds over the candidates, the first of them untimed: at least three
-    // timed ones, and up to eight until a candidate's take 2 ms together.  A
-    // candidate that the first timed round has a tenth behind drops out.
+    // timed ones, and up to eight until the fastest candidate's take 2 ms.  A
+    // candidate whose better one of the first two is a tenth behind drops out.
     cudaError_t err = cudaSuccess;
     for (int round = 0; err == cudaSuccess; ++round) {
       for (Candidate &c : cand) {
@@ -1006,19 +1012,24 @@ template <typename S> class EngineT : public Engine {
         if (err == cudaSuccess) err = cudaEventRecord(e1, st);
         if (err == cudaSuccess) err = cudaEventSynchronize(e1);
         if (err == cudaSuccess) err = cudaEventElapsedTime(&one, e0, e1);
-        if (round > 0) c.ms += one;
+        if (round > 0) c.ms.push_back(one);
       }
-      if (round == 0 || err != cudaSuccess) continue;
-      std::stable_sort(cand.begin(), cand.end(),
-                       [](const Candidate &x, const Candidate &y) { return x.ms < y.ms; });
-      if (round == 1)
-        while (cand.back().ms > 1.1f * cand.front().ms) cand.pop_back();
-      if (cand.size() == 1 || (round >= 3 && cand.front().ms >= 2.0f) || round == 8) break;
+      if (round < 2) continue;
+      float least = 1e30f;
+      for (const Candidate &c : cand) least = std::min(least, c.least());
+      if (round == 2)
+        cand.erase(std::remove_if(cand.begin(), cand.end(),
+                                  [&](const Candidate &c) { return c.least() > 1.1f * least; }),
+                   cand.end());
+      if (cand.size() == 1 || (round > 2 && least * round >= 2.0f) || round == 8) break;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     CUDA_TRY(err);
-    const Candidate best = cand.front();
+    const Candidate &best =
+        *std::min_element(cand.begin(), cand.end(), [](const Candidate &x, const Candidate &y) {
+          return x.mean() < y.mean();
+        });
     if (!batch_form) {
       tile_rows_ = best.form;
       form_tuned_ = true;
