@@ -981,7 +981,7 @@ template <typename S> class EngineT : public Engine {
     };
     std::vector<Candidate> cand;
     for (int rows : forms)
-      for (int ch : chunks) cand.push_back({rows, ch, 0.0f});
+      for (int ch : chunks) cand.push_back({rows, ch, {}});
     auto stages = [&](const Candidate &c) {
       for (int irk = 0; irk < 3; ++irk) {
         int fb[3];
