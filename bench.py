@@ -303,7 +303,7 @@ def _setup_scenario(cgfdm, w, prec):
 
 def _sim_of(cgfdm, setup, prec, nt, device):
     """A handle of one scenario; its tile form and work-item depth are the
-    autotuner's (alone), or its depth for the 32 x 16 form (in a batch)."""
+    autotuner's (alone), or its depth for the 32 x 8 form (in a batch)."""
     d0 = setup["desc"]
     sim = cgfdm.Simulation(cgfdm.make_desc(d0.nx, d0.ny, d0.nz, d0.npml, d0.dh, d0.dt, nt, prec,
                                            cgfdm.KERNEL_AUTO, device))
@@ -867,6 +867,8 @@ def main():
                        "grid": [desc0.nx, desc0.ny, desc0.nz], "points": npts,
                        "kernel": args.kernel, "tile_form": form, "chunk_planes": chunk,
                        "surface_kernel": "tiled" if fast_top else "exact-order",
+                       "stage_launches": "in turn, with events between them; a run without "
+                                         "timing (e2e) overlaps a stage's launches",
                        "parallelism": "replicas" if ws > 1 else "single",
                        "l2": "inputs larger than L2 (%.2f GB per wavefield buffer), no flush" % (
                            9 * (desc0.nx + 6) * (desc0.ny + 6) * (desc0.nz + 6) *

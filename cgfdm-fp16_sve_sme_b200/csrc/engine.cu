@@ -605,8 +605,8 @@ template <typename S> class EngineT : public Engine {
   // Checkpoint at a step boundary, raw device contents: a header, the three
   // stage buffers A, X, Y (A is the step state; X and Y keep point-source
   // values in their halo cells), the step-start PML auxiliaries, the PGV map,
-  // the seismograms and the step counter.  T and the other auxiliary buffers
-  // are rewritten by the next stage 0 before they are read.
+  // the seismograms and the step counter.  The next step writes T and the
+  // other auxiliary buffers before it reads them.
   struct CkptHeader {
     char magic[8];
     int32_t precision, nx, ny, nz, npml, nt, nsta, it;
@@ -1047,7 +1047,7 @@ template <typename S> class EngineT : public Engine {
     last_out_ = a.wout;
     last_aux_out_ = aux_total_ > 0 ? auxbuf(out_of[irk]) : nullptr;
     // events per timed stage: [0] start, [1] after the streaming kernel,
-    // [2] before the exact-order kernel, [3] end (after the exact-order kernel)
+    // [2] before the surface kernel, [3] end (after it)
     cudaEvent_t *ev = nullptr;
     if (timing_) {
       while ((int)stage_ev_.size() < 4 * (stage_used_ + 1)) {
@@ -1142,8 +1142,9 @@ template <typename S> class EngineT : public Engine {
 
   // The coefficient upload stages the host fields through the RK accumulator
   // T, a few fields at a time, instead of allocating a staging buffer as
-  // large as the model: outside a stage T is free (every stage 0 rewrites it
-  // before anything reads it).  T is cleared afterwards.
+  // large as the model: between steps T is free (a whole step writes it in
+  // stage 2, a stage 0 by itself at once, before anything reads it).  T is
+  // cleared afterwards.
   cudaError_t upload_through_accumulator(const float *src, S *dst, int nfield) {
     const size_t tbytes = sizeof(S) * 9 * (size_t)g_.L.fs;
     const int per = (int)std::min<size_t>((size_t)nfield, tbytes / (sizeof(float) * (size_t)g_.num));
@@ -1275,8 +1276,9 @@ namespace {
 // Several handles of one precision advanced together: per step, each
 // member's sources; per stage, the streaming part of all members in
 // persistent launches whose work queue spans them (members grouped by their
-// MacCormack signs, which depend on each member's own step), then each
-// member's free-surface layers; then stations / PGV.  A step can be
+// MacCormack signs, which depend on each member's own step, and by the kind of
+// grid) and beside them the free-surface layers of up to kSurfBatch members a
+// launch; then each member's stations / PGV.  A step can be
 // replayed as a CUDA graph (per phase of the batch's step count mod 8, since
 // every member's signs repeat with period 8).
 template <typename S> class BatchT : public BatchBase {

@@ -35,7 +35,7 @@ constexpr int kStreamMapsBytes = 3072;
 // two x-adjacent points per thread.
 constexpr int kTilePair = 64;
 // `after_main` (optional) is recorded right after the streaming kernel,
-// before the exact-order kernel; `nlaunch` (optional) is increased by the
+// before the surface kernel; `nlaunch` (optional) is increased by the
 // number of kernels launched; `tile_rows` selects the tile form: 16 (32 x 16
 // tiles, one CTA per SM), 8 (32 x 8, two CTAs per SM) or kTilePair (16-bit
 // storage: the paired-point kernel on 64 x 8 interior tiles, the 32 x 8 PML

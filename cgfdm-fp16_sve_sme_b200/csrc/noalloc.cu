@@ -166,9 +166,14 @@ int stage_noalloc(const cgfdm_stage_buffers &b, cudaStream_t st, unsigned char *
     StageArgs<S> lower = a;
     lower.kbeg = HALO;
     lower.kend = ksurf;
-    // the fastest tile form of most grids (all forms give the same bits):
-    // 225x225x201 FP32 2.78 -> 2.66 ms a step, 201x161x121
-    // FP16 1.35 -> 1.16 ms, against 32 x 16 tiles
+    // All forms give the same bits.  Measured, ms a step: 225x225x201 FP32
+    // 2.66 in 32 x 8 tiles, 2.78 in 32 x 16.  FP16 with a 12-cell PML, paired
+    // against 32 x 8: 0.445 / 0.547 at 96x96x100, 0.989 / 1.089 at 107x200x150
+    // (no paired interior there: all of it runs the PML variant), 0.835 / 0.809
+    // at 120x120x100, 1.157 / 1.156 at 201x161x121, 2.884 / 3.064 at
+    // 601x301x100.  Without a PML the paired form is ahead on wide grids only:
+    // 1.989 / 2.036 at 401x401x100, 0.866 / 0.816 at 225x187x133, 0.488 / 0.350
+    // at 64x300x100.
     NA_TRY(launch_stage_stream<S>(lower, maps, err, counter, StreamPair{st, st}, nullptr, nullptr,
                                   sizeof(S) == 2 ? kTilePair : 8));
   }

@@ -2,8 +2,9 @@
 // translation unit per storage type (stage_stream_f32.cu, _f16.cu, _bf16.cu),
 // each instantiating its own kernels.
 //
-// Persistent CTAs (one 512-thread CTA per SM) pull work items from an atomic
-// queue; an item is a 32 x 16 column tile and a chunk of z planes, ordered so
+// Persistent CTAs (one of 512 threads an SM with 32 x 16 tiles, two of 256 with
+// 32 x 8) pull work items from an atomic
+// queue; an item is a column tile and a chunk of z planes, ordered so
 // that concurrently running items are neighbours at the same depth (their
 // halo rows meet in L2).  Within an item the CTA sweeps z against the
 // MacCormack z direction (upward when FB3 = -1, downward when FB3 = +1), so
@@ -11,12 +12,13 @@
 // it: a 5-plane register window per thread holds the z stencil, and shared
 // memory holds three rings fed by 4-D TMA tile loads (cp.async.bulk.tensor,
 // no multicast), each slot guarded by an mbarrier:
-//   W ring (4): the 9 wavefield components of one input plane with the x/y
-//               halo of the one-sided stencils (x origin 16-byte aligned);
-//   C ring (2): the 9 metrics and (mu, lambda, buoyancy) of one output plane;
-//   M ring (2): the RK step state m and accumulator t (or what t is formed
-//               from) of one output plane (stages that read them);
-// (the depths are those of FP32 in 32 x 16 tiles, see Rings).
+//   W ring: the 9 wavefield components of one input plane with the x/y
+//           halo of the one-sided stencils (x origin 16-byte aligned);
+//   C ring: the metrics and (mu, lambda, buoyancy) of one output plane;
+//   M ring: the RK step state m and accumulator t (or what t is formed
+//           from) of one output plane (stages that read them);
+// (3 to 5, 2 to 3 and 2 to 3 planes by storage, tile and stage class, see
+// Rings).
 // With 16-bit storage the interior variant converts each W plane to FP32 once
 // in shared memory (two plane buffers), so its stencils read FP32 like the
 // FP32 kernel instead of converting every tap.
@@ -33,7 +35,7 @@
 // sums use the bare MacCormack weights, and each direction's elastic
 // combination is formed once and scaled by the sign FB, 1/DH and the PML beta
 // (main update) or d (auxiliary update), equal to the reference up to
-// rounding.  The three free-surface layers are left to the exact-order kernel.
+// rounding.  The three free-surface layers are left to the surface kernel.
 //
 // Every mbarrier wait is bounded (2^31 clock cycles); on expiry the CTA sets
 // the error flag, drains the copies it issued (again bounded) and returns.
@@ -421,7 +423,7 @@ struct MapSet {
 
 // Work items of one launch.  The z range [kbeg, kend) is cut at kz, the top
 // of the bottom PML slab: nzc chunks of chunk_p planes below it and nic
-// chunks of chunk_i planes above it.  Tiles are 32 x 16 columns on an
+// chunks of chunk_i planes above it.  Tiles are 32 x 16 or 32 x 8 columns on an
 // ntx x nty grid; tiles [bx_lo, bx_hi) x [by_lo, by_hi) touch no x or y PML
 // slab.  The interior launch covers interior tiles x upper chunks; the PML
 // launch covers every tile of the lower chunks and the edge tiles (all
@@ -1543,7 +1545,7 @@ template <typename S, int FB1, int FB2, int FB3, int RK, bool VT>
 cudaError_t launch_batch(const StageArgs<S> *args, const void *const *maps, int n, int *err,
                          int *counter, StreamPair st, int *nlaunch) {
   const int nsm = sm_count();
-  // the launch parameters (about 19 KB) are assembled in per-thread storage
+  // the launch parameters (about 23 KB) are assembled in per-thread storage
   static thread_local BatchParams<S> params;
   BatchParams<S> *bp = &params;
   for (int b0 = 0; b0 < n; b0 += kBatchMax) {

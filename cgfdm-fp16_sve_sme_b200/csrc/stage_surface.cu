@@ -20,6 +20,9 @@
 // the exact-order kernel on the slab columns): 64x64x48 40-80 -> 13.5 us,
 // 401x401x201 with a 20-cell PML 90-168 -> 61-72 us, 601x601x401 145-263 ->
 // 125-149 us (FP32, cold cache).
+// At 128 registers the single-scenario form has no spills; the form for several
+// scenarios spills (a 72-byte frame, 144 bytes of stores and 72 of loads a
+// thread).
 // FP32 arithmetic with FMA contraction, equal to the reference up to rounding.
 #include <algorithm>
 

@@ -99,7 +99,12 @@ int cgfdm_destroy(cgfdm_handle *h);
 /* Uploads the medium/metric coefficients and free-surface matrices in the
  * reference layout (the CJM and mat_rDZ arguments of propagate()).  Waits for
  * the handle's outstanding work first and returns once the upload is done;
- * the RK accumulator is cleared (a stage 0 rewrites it before any read). */
+ * the RK accumulator is cleared (the next step writes it before any read).
+ * If xi_y, xi_z, eta_x and eta_z are zero in every cell (a grid stretched in z
+ * only), cgfdm_run and batches leave out the terms that these multiply.  For
+ * finite fields the results are the same bits; an infinity or NaN in the
+ * wavefield then spreads through the other metrics' terms only, not through
+ * zero times infinity. */
 int cgfdm_set_model(cgfdm_handle *h, const float *cjm, const float *rdz);
 
 /* The smoothed explosive point source of singleSource.cpp:78-177 at padded
@@ -165,7 +170,8 @@ int cgfdm_aux_floats(cgfdm_handle *h, int64_t *n);   /* floats of one aux set */
 /* Device timing of the last cgfdm_run, from CUDA events on its stream (only
  * when enabled with cgfdm_set_timing): [0] the whole run in ms, [1] the sum
  * of the fused-stage kernel durations in ms, [2] the number of those stage
- * launches. */
+ * launches.  While it is enabled the launches of a stage run in turn, to time
+ * each; otherwise they overlap, so that a run is faster than timed. */
 int cgfdm_set_timing(cgfdm_handle *h, int32_t on);
 int cgfdm_get_timing(cgfdm_handle *h, float *ms3);
 
@@ -174,24 +180,24 @@ int cgfdm_get_timing(cgfdm_handle *h, float *ms3);
  * bytes those launches move (fields read and written once per point and
  * stage; the PML auxiliaries, handled inside the same kernel, are not
  * counted), [3] kernels launched by the run (counted whether or not timing is
- * on), [4] time between the streaming kernel and the exact-order kernel in
- * ms (no kernel runs there), [5] exact-order (free-surface) kernel time in
- * ms, [6] stages timed, [7] the streaming kernel's tile height (0: not used). */
+ * on), [4] time between the streaming kernel and the surface kernel in ms (no
+ * kernel runs there), [5] free-surface (or exact-order) kernel time in ms, [6] stages timed, [7] the streaming kernel's tile height (0: not used). */
 int cgfdm_get_kernel_stats(cgfdm_handle *h, double *out8);
 
 /* Tile form of the streaming kernel: 16 (32 x 16 tiles, one CTA per SM),
  * 8 (32 x 8 tiles, two CTAs per SM), 64 (FP16 / BF16 storage only: 64 x 8
  * interior tiles with two x-adjacent points per thread, the 32 x 8 form
- * elsewhere), or 0 (the default): autotune -- the first cgfdm_run times one
- * stage with each form on this handle's buffers (blocking that call for a
- * few stage times) and keeps the fastest; the choice is cached per
- * (precision, grid) for the process.  If the environment variable
- * CGFDM_TUNE_CACHE names a file, choices are also kept there across
- * processes: a grid with an entry for this GPU is not timed again, and new
- * choices are written back (a JSON object of [form, depth, tiled surface]
- * triples; a malformed file is ignored and rewritten).  The forms split the grid differently
- * between the interior launch and the PML launch, whose variants round the
- * elastic combination differently, so they agree to rounding. */
+ * elsewhere), or 0 (the default): autotune -- the first cgfdm_run times
+ * stages 0 to 2 of a step with each form and several item depths on this
+ * handle's buffers (blocking that call for some tens of stage times) and keeps
+ * the fastest.  The choice is kept for the process under the device,
+ * precision, grid, PML width and kind of grid (stretched in z only or
+ * general); a cgfdm_set_model of the other kind makes the next cgfdm_run
+ * choose again.  If the environment variable CGFDM_TUNE_CACHE names a file,
+ * choices are also kept there across processes: a grid with an entry for this
+ * GPU and this revision of the kernels is not timed again, and new choices
+ * are written back (a JSON object of [form, depth, tiled surface] triples; a
+ * malformed file is ignored and rewritten).  All forms give the same bits. */
 int cgfdm_set_tile_rows(cgfdm_handle *h, int32_t rows);
 
 /* Depth of the streaming kernel's work items: the planes above the bottom
@@ -247,9 +253,11 @@ int cgfdm_set_graph(cgfdm_handle *h, int32_t on);
  * sources, stations, and step counters).  cgfdm_batch_run advances every
  * member by nsteps: per stage, the streaming part of all members runs in
  * persistent launches whose work queue spans the members (16 members per
- * launch pair; members at different phases of the MacCormack schedule are
- * grouped), and each member's free-surface layers, sources and stations run
- * as its own small kernels.  Results equal running each member alone.  With
+ * launch pair; members at different phases of the MacCormack schedule or of
+ * the other kind of grid are grouped apart), the free-surface layers of up to
+ * 16 members share a launch, and each member's sources and stations run as its
+ * own small kernels.  Results equal running each member alone, also when a
+ * member advances by itself between two runs of the batch.  With
  * cgfdm_batch_set_graph(b, 1) each batch step is replayed as a CUDA graph.
  * Members keep their own state: read their results with the handle getters
  * after cgfdm_batch_synchronize.  Destroy the batch before its members. */

@@ -102,8 +102,8 @@ def test_noalloc_stage_matches_handle_stage(gpu_available, precision, case, grid
     cjm, rdz = _model(NX, NY, NZ, kind)
     st = _state(p, 100 + case, kind)
 
-    # the existing entry point: a handle and cgfdm_stage (tile height 16, the
-    # form the no-allocation stage launches)
+    # the existing entry point: a handle and cgfdm_stage (in 32 x 16 tiles; all
+    # tile forms give the same bits)
     d = cgfdm.make_desc(NX, NY, NZ, NPML, 100.0, 0.008, 1, prec, cgfdm.KERNEL_AUTO)
     with cgfdm.Simulation(d) as sim:
         sim.set_tile_rows(16)
